@@ -110,6 +110,8 @@ struct KParams {
   // (A, C) of node npost_node
   float *npost;
   int npost_node;
+  // (R,) 1 for leaves
+  const uint8_t *leaf;
   // branch joint posteriors (k_tree4, A = 4): (R, 4, 4, C) or the (4, 4, C)
   // of node npost_node
   float *bpost;
@@ -136,6 +138,34 @@ int big_acc_group(int A);
 // mode: 0 inside pass only (LogLike / RootProb), 1 stage eigen vectors, 2 stage F81 vectors
 int launch_walk(const KParams &p, int A, int mode, bool tc, float *sa, float *sb, int c_base, int c_count,
                 int grid, cudaStream_t s);
+// four-lane walk (k_qwalk.cu): inside pass only, or with the raw staging
+// (flags: kQLeafU also stages the leaves' U, kQRotate rotates a row's chunks
+// by stage_rot).  f81: the F81 / JC closed form (any A; the general
+// products: A = 16, 20, 32).
+enum : int { kQLeafU = 1, kQRotate = 2 };
+struct QGrid {
+  int variant;            // columns per lane
+  int grid;
+  size_t slot_bytes;      // slot vectors and words of the whole grid
+  size_t vec_bytes;       // offset of the words within them
+};
+bool qwalk_supported(int A, bool f81);
+int qwalk_grid(int A, bool f81, bool outside, int C, int nslots, int nsm, QGrid *g);
+int launch_qwalk(const KParams &p, int A, bool f81, bool outside, float *sa, float *sb, int flags, int c_base,
+                 int c_count, const QGrid &g, cudaStream_t s);
+// A = 16, 20, 32: k_qwalk's raw staging into the eigenbasis, in place
+// (k_proj.cu); vd, vu: the FP32 projection matrices (host)
+bool proj_supported(int A);
+int launch_proj(const KParams &p, int A, const float *vd, const float *vu, float *sa, float *sb, int c_base,
+                int c_count, int nsm, cudaStream_t s);
+// Rotation of the 16-byte chunks of a staged row of column c (kQRotate), and
+// the float offset of chunk k under it: rows whose length is a multiple of
+// 16 floats start on the same banks.
+__host__ __device__ constexpr int stage_rot(int A, int c) { return A == 16 ? c >> 1 : A == 32 ? c : 0; }
+template <int A>
+__host__ __device__ constexpr int stage_chunk(int k, int rot) {
+  return (A == 16 || A == 32) ? 4 * ((k + rot) & (A / 4 - 1)) : 4 * k;
+}
 // the walk of the posteriors (k_walkpost.cu) at A = 4, 8 and the large
 // alphabets: mode 0 (inside only: the root's posterior) or 3 (node
 // posteriors, and D_n s_n, U_n staged in the original basis when sa is given)

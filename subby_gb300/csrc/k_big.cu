@@ -277,8 +277,9 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const int cc = grp * 8 + q;
-            const float4 d = *reinterpret_cast<const float4 *>(da + cc * A + k0);
-            const float4 u = *reinterpret_cast<const float4 *>(db + cc * A + l0);
+            // (rot(cc) = rot(q): the groups of 8 columns start at rotation 0)
+            const float4 d = *reinterpret_cast<const float4 *>(da + cc * A + stage_chunk<A>(k0 / 4, stage_rot(A, q)));
+            const float4 u = *reinterpret_cast<const float4 *>(db + cc * A + stage_chunk<A>(l0 / 4, stage_rot(A, q)));
             const float dk[4] = {d.x, d.y, d.z, d.w};
             const float2 up[2] = {make_float2(u.x, u.y), make_float2(u.z, u.w)};
 #pragma unroll

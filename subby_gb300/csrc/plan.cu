@@ -249,9 +249,13 @@ struct subby_plan {
   int nslots = 0;
   // tree program of k_tree (stored / derived node classification), and the
   // walk's program with every internal node stored
-  std::vector<int4> prog, prog_w;
-  int prog_steps = 0, prog_slots = 0, prog_w_steps = 0, prog_w_slots = 0;
-  int4 *d_prog = nullptr, *d_prog_w = nullptr;
+  // prog_s: the same steps for inside-only walks, with a slot reused as soon
+  // as its parent has read it
+  std::vector<int4> prog, prog_w, prog_s;
+  int prog_steps = 0, prog_slots = 0, prog_w_steps = 0, prog_w_slots = 0, prog_s_slots = 0;
+  int4 *d_prog = nullptr, *d_prog_w = nullptr, *d_prog_s = nullptr;
+  uint8_t *d_leaf = nullptr;          // (R,) 1 for leaves
+  std::vector<float> hVd, hVu;        // FP32 projection matrices (kernel parameters of k_proj)
   std::vector<double> V, mu, pi, t;   // FP64 model and branch lengths (host)
   float f81_mu = 0.f;
   int f81_model = 0;   // M(t) has the F81 / JC closed form (checked on the host)
@@ -487,6 +491,22 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
   };
   build_prog(false, P->prog, P->prog_steps, P->prog_slots);
   build_prog(true, P->prog_w, P->prog_w_steps, P->prog_w_slots);
+  {
+    // postorder evaluation stack: a node takes the slot of its first stored child
+    P->prog_s = P->prog_w;
+    std::vector<int> at(R, -1);
+    int sp = 0;
+    for (size_t i = 0; i < P->prog_s.size(); i += 4) {
+      int4 &own = P->prog_s[i], &l = P->prog_s[i + 1], &r = P->prog_s[i + 2];
+      l.y = l.y >= 0 ? at[l.x] : l.y;
+      r.y = r.y >= 0 ? at[r.x] : r.y;
+      sp -= (l.y >= 0) + (r.y >= 0);
+      if (!own.z) {
+        at[own.x] = own.y = sp++;
+        P->prog_s_slots = std::max(P->prog_s_slots, sp);
+      }
+    }
+  }
 
   // ---- FP64 host tables
   P->t.assign(dist, dist + R);
@@ -632,8 +652,18 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(P->d_prog_w, P->prog_w.data(), sizeof(int4) * P->prog_w.size(), cudaMemcpyHostToDevice,
                           qs);
+    if (e == cudaSuccess) e = pool_alloc((void **)&P->d_prog_s, sizeof(int4) * P->prog_s.size(), P->pool, qs);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(P->d_prog_s, P->prog_s.data(), sizeof(int4) * P->prog_s.size(), cudaMemcpyHostToDevice,
+                          qs);
+    std::vector<uint8_t> leaf((size_t)R);
+    for (int n = 0; n < R; ++n) leaf[n] = left[n] < 0;
+    if (e == cudaSuccess) e = pool_alloc((void **)&P->d_leaf, leaf.size(), P->pool, qs);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(P->d_leaf, leaf.data(), leaf.size(), cudaMemcpyHostToDevice, qs);
     if (e != cudaSuccess) return cleanup(cuda_fail(e, "program upload"));
   }
+  P->hVd.assign(hsm.begin() + (o.Vd - o.Vu), hsm.begin() + (o.Vd - o.Vu) + A * A);
+  P->hVu.assign(hsm.begin(), hsm.begin() + A * A);
   std::vector<float> hMT, hMN, hGQ;
   std::vector<float2> hcx;
   std::vector<int> grp_br;
@@ -869,7 +899,7 @@ int subby_plan_destroy(subby_plan *P) {
   if (s && P->used) cudaStreamWaitEvent(s, P->last_use, 0);
   if (P->s_in) cudaStreamSynchronize(P->s_in);
   if (P->s_out) cudaStreamSynchronize(P->s_out);
-  void *bufs[] = {P->d_tab, P->d_tab64, P->d_steps, P->d_slots, P->d_prog, P->d_prog_w, P->d_tab16, P->d_err,
+  void *bufs[] = {P->d_tab, P->d_tab64, P->d_steps, P->d_slots, P->d_prog, P->d_prog_w, P->d_prog_s, P->d_leaf, P->d_tab16, P->d_err,
                   P->d_cx, P->d_grp_br, P->d_gq};
   for (void *b : bufs)
     if (b) cudaFreeAsync(b, s);
@@ -1224,10 +1254,52 @@ KParams walk_params(const subby_plan *P, const int32_t *d_aln, int C, int mode, 
   k.noderiv = all ? 1 : 0;
   k.nsteps = all ? P->prog_w_steps : P->prog_steps;
   k.nslots = std::max(all ? P->prog_w_slots : P->prog_slots, 1);
+  k.leaf = P->d_leaf;
   k.tab16 = P->d_tab16;
   k.err = P->d_err;
   k.dbg_wait_polls = g_dbg_wait_polls.load();
   return k;
+}
+
+// Scratch of the walk: which kernel, its grid and the bytes of its slots.
+// q: the four-lane walk (k_qwalk) — raw staging or inside only at A = 16, 20,
+// 32, and at A = 64 the F81 / JC closed form; otherwise k_walk.
+struct WalkPlan {
+  bool q = false, f81 = false, outside = false;
+  QGrid g{};
+  int grid = 1;
+  size_t vec_bytes = 0, word_bytes = 0;
+};
+size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+int plan_walk(const subby_plan *P, KParams &k, bool q, bool outside, int chunk, int per_sm, WalkPlan *w) {
+  w->outside = outside;
+  w->f81 = P->f81_model != 0;
+  w->q = q && qwalk_supported(P->A, w->f81);
+  if (w->q) {
+    // every internal node stored; inside only: slots reused bottom-up
+    k.prog = outside ? P->d_prog_w : P->d_prog_s;
+    k.noderiv = 1;
+    k.nsteps = P->prog_w_steps;
+    k.nslots = std::max(outside ? P->prog_w_slots : P->prog_s_slots, 1);
+    if (qwalk_grid(P->A, w->f81, outside, chunk, k.nslots, P->nsm, &w->g) != 0)
+      return fail(SUBBY_ERR_UNSUPPORTED, "walk: unsupported alphabet");
+    w->vec_bytes = al256(w->g.vec_bytes);
+    w->word_bytes = al256(w->g.slot_bytes - w->g.vec_bytes);
+    return 0;
+  }
+  const int tile = big_tile();
+  w->grid = std::max(1, std::min((chunk + tile - 1) / tile, P->nsm * per_sm));
+  w->vec_bytes = al256((size_t)w->grid * k.nslots * tile * P->A * sizeof(float));
+  w->word_bytes = al256((size_t)w->grid * k.nslots * tile * 2 * sizeof(int));  // a word per column half
+  return 0;
+}
+
+// The walk's slots at the start of the workspace; returns what follows them.
+char *place_walk(KParams &k, const WalkPlan &w, void *base) {
+  k.scrV = (float *)base;
+  k.scrW = (int *)((char *)base + w.vec_bytes);
+  return (char *)base + w.vec_bytes + w.word_bytes;
 }
 
 int run_big(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_counts, float *d_root,
@@ -1242,6 +1314,10 @@ int run_big(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_
   const int tile = big_tile();
   const int H = (A + 31) / 32;
   const bool counts = (mode & kModeCounts) != 0 && R > 1;
+  const bool eigen = counts && !(mode & kModeF81);
+  // raw staging by the four-lane walk, projected by k_proj; A = 64 keeps the
+  // eigen staging of k_walk
+  const bool quad = g_kernel_sel != 1 && (proj_supported(A) || !eigen);
   // chunk of columns (multiple of the tile) bounded by the staging budget
   int chunk = C;
   if (counts) {
@@ -1253,29 +1329,18 @@ int run_big(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_
     const size_t even = ((size_t)C + nch - 1) / nch;
     chunk = (int)std::min<size_t>((size_t)C, (even + tile - 1) / tile * tile);
   }
-  const int walk_grid = std::max(1, std::min((chunk + tile - 1) / tile, P->nsm * (H == 2 ? 1 : 2)));
-  const size_t slot_floats = (size_t)walk_grid * k.nslots * tile * A;
-  const size_t slot_ints = (size_t)walk_grid * k.nslots * tile * 2;  // a word per column half
-  const size_t stage_floats = counts ? (size_t)(R - 1) * chunk * A : 0;
+  WalkPlan w;
+  int rc;
+  if ((rc = plan_walk(P, k, quad, counts, chunk, H == 2 ? 1 : 2, &w))) return rc;
+  const size_t stage_bytes = counts ? al256((size_t)(R - 1) * chunk * A * sizeof(float)) : 0;
   // A = 64 F81 counts on the tensor cores: per-branch scalars staged too
   const bool f81tc = counts && (mode & kModeF81) && tc && !(mode & kModeBranch);
-  const size_t stage_c_floats = f81tc ? (size_t)(R - 1) * chunk * 2 : 0;
-  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  int rc;
-  if ((rc = P->grow(P->work,
-                    al(slot_floats * 4) + al(slot_ints * 4) + 2 * al(stage_floats * 4) + al(stage_c_floats * 4) + 256,
-                    stream)))
-    return rc;
-  char *base = (char *)P->work.p;
-  k.scrV = (float *)base;
-  base += al(slot_floats * 4);
-  k.scrW = (int *)base;
-  base += al(slot_ints * 4);
+  const size_t stage_c_bytes = f81tc ? al256((size_t)(R - 1) * chunk * sizeof(float2)) : 0;
+  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * stage_bytes + stage_c_bytes + 256, stream))) return rc;
+  char *base = place_walk(k, w, P->work.p);
   float *sa = (float *)base;
-  base += al(stage_floats * 4);
-  float *sb = (float *)base;
-  base += al(stage_floats * 4);
-  k.stage_c = f81tc ? (float2 *)base : nullptr;
+  float *sb = (float *)(base + stage_bytes);
+  k.stage_c = f81tc ? (float2 *)(base + 2 * stage_bytes) : nullptr;
   const int wmode = counts ? ((mode & kModeF81) ? 2 : 1) : 0;
   if (!counts && (mode & kModeCounts)) {
     // a single-node tree has no branch: counts are zero
@@ -1284,10 +1349,16 @@ int run_big(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_
   }
   for (int c0 = 0; c0 < C; c0 += chunk) {
     const int cc = std::min(chunk, C - c0);
-    int lr = launch_walk(k, A, wmode, tc, sa, sb, c0, cc, walk_grid, stream);
+    int lr = w.q ? launch_qwalk(k, A, w.f81, counts, sa, sb, eigen ? kQRotate : kQLeafU, c0, cc, w.g, stream)
+                 : launch_walk(k, A, wmode, tc, sa, sb, c0, cc, w.grid, stream);
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("walk launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
     if (counts) {
+      if (w.q && eigen) {
+        lr = launch_proj(k, A, P->hVd.data(), P->hVu.data(), sa, sb, c0, cc, P->nsm, stream);
+        if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("projection launch failed: ") + cudaGetErrorString((cudaError_t)lr));
+        g_launches += 1;
+      }
       const int G = big_acc_group(A);
       const long long items = (long long)(cc + G - 1) / G * ((mode & kModeBranch) ? (R - 1) : 1);
       const int agrid = (int)std::max<long long>(1, std::min<long long>(items, P->nsm));
@@ -1360,27 +1431,22 @@ int run_post(subby_plan *P, const int32_t *d_aln, int C, int node, float *d_node
     chunk = (int)std::min<size_t>((size_t)C, (even + tile - 1) / tile * tile);
   }
   const int per_sm = A <= 8 ? 8 : (H == 2 ? 1 : 2);
-  const int walk_grid = std::max(1, std::min((chunk + tile - 1) / tile, P->nsm * per_sm));
-  const size_t slot_floats = (size_t)walk_grid * k.nslots * tile * A;
-  const size_t slot_ints = (size_t)walk_grid * k.nslots * tile * 2;  // a word per column half
-  const size_t stage_floats = stage ? (size_t)(R - 1) * chunk * A : 0;
-  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  WalkPlan w;
   int rc;
-  if ((rc = P->grow(P->work, al(slot_floats * 4) + al(slot_ints * 4) + 2 * al(stage_floats * 4) + 256, stream)))
+  if ((rc = plan_walk(P, k, !(outside && d_node), outside, chunk, per_sm, &w))) return rc;
+  const size_t stage_floats = stage ? (size_t)(R - 1) * chunk * A : 0;
+  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + 256, stream)))
     return rc;
-  char *base = (char *)P->work.p;
-  k.scrV = (float *)base;
-  base += al(slot_floats * 4);
-  k.scrW = (int *)base;
-  base += al(slot_ints * 4);
+  char *base = place_walk(k, w, P->work.p);
   float *sa = stage ? (float *)base : nullptr;
-  base += al(stage_floats * 4);
+  base += al256(stage_floats * 4);
   float *sb = stage ? (float *)base : nullptr;
   const int n_lo = all ? 1 : node, n_hi = all ? R : node + 1;
   const int row_off = all ? 0 : node;
   for (int c0 = 0; c0 < C; c0 += chunk) {
     const int cc = std::min(chunk, C - c0);
-    int lr = launch_walk_post(k, A, outside ? 3 : 0, tc, sa, sb, c0, cc, walk_grid, stream);
+    int lr = w.q ? launch_qwalk(k, A, w.f81, outside, sa, sb, kQLeafU, c0, cc, w.g, stream)
+                 : launch_walk_post(k, A, outside ? 3 : 0, tc, sa, sb, c0, cc, w.grid, stream);
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("walk launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
     if (!stage) continue;
@@ -1427,30 +1493,25 @@ int run_cx(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_c
     chunk = (int)std::min<size_t>((size_t)C, (even + tile - 1) / tile * tile);
   }
   const int per_sm = A <= 8 ? 8 : (H == 2 ? 1 : 2);
-  const int walk_grid = std::max(1, std::min((chunk + tile - 1) / tile, P->nsm * per_sm));
-  const size_t slot_floats = (size_t)walk_grid * k.nslots * tile * A;
-  const size_t slot_ints = (size_t)walk_grid * k.nslots * tile * 2;  // a word per column half
+  WalkPlan w;
+  int rc;
+  if ((rc = plan_walk(P, k, true, counts, chunk, per_sm, &w))) return rc;
   const size_t stage_floats = counts ? (size_t)(R - 1) * chunk * A : 0;
   const size_t cbuf_bytes = (counts && bt64) ? (size_t)chunk * A * A * sizeof(float2) : 0;
-  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  int rc;
-  if ((rc = P->grow(P->work, al(slot_floats * 4) + al(slot_ints * 4) + 2 * al(stage_floats * 4) + al(cbuf_bytes) + 256,
+  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + al256(cbuf_bytes) + 256,
                     stream)))
     return rc;
-  char *base = (char *)P->work.p;
-  k.scrV = (float *)base;
-  base += al(slot_floats * 4);
-  k.scrW = (int *)base;
-  base += al(slot_ints * 4);
+  char *base = place_walk(k, w, P->work.p);
   float *sa = counts ? (float *)base : nullptr;
-  base += al(stage_floats * 4);
+  base += al256(stage_floats * 4);
   float *sb = counts ? (float *)base : nullptr;
-  base += al(stage_floats * 4);
+  base += al256(stage_floats * 4);
   float2 *cbuf = cbuf_bytes ? (float2 *)base : nullptr;
   const int G = cx_columns_per_cta(A);
   for (int c0 = 0; c0 < C; c0 += chunk) {
     const int cc = std::min(chunk, C - c0);
-    int lr = launch_walk_post(k, A, counts ? 3 : 0, tc, sa, sb, c0, cc, walk_grid, stream);
+    int lr = w.q ? launch_qwalk(k, A, w.f81, counts, sa, sb, kQLeafU, c0, cc, w.g, stream)
+                 : launch_walk_post(k, A, counts ? 3 : 0, tc, sa, sb, c0, cc, w.grid, stream);
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("walk launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
     if (!counts) continue;
@@ -1564,25 +1625,20 @@ int run_cx_grad(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, const
     chunk = (int)std::min<size_t>((size_t)C, (even + tile - 1) / tile * tile);
   }
   const int per_sm = A <= 8 ? 8 : (H == 2 ? 1 : 2);
-  const int walk_grid = std::max(1, std::min((chunk + tile - 1) / tile, P->nsm * per_sm));
-  const size_t slot_floats = (size_t)walk_grid * k.nslots * tile * A;
-  const size_t slot_ints = (size_t)walk_grid * k.nslots * tile * 2;  // a word per column half
-  const size_t stage_floats = R > 1 ? (size_t)(R - 1) * chunk * A : 0;
-  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  WalkPlan w;
   int rc;
-  if ((rc = P->grow(P->work, al(slot_floats * 4) + al(slot_ints * 4) + 2 * al(stage_floats * 4) + 256, stream)))
+  if ((rc = plan_walk(P, k, true, R > 1, chunk, per_sm, &w))) return rc;
+  const size_t stage_floats = R > 1 ? (size_t)(R - 1) * chunk * A : 0;
+  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + 256, stream)))
     return rc;
-  char *base = (char *)P->work.p;
-  k.scrV = (float *)base;
-  base += al(slot_floats * 4);
-  k.scrW = (int *)base;
-  base += al(slot_ints * 4);
+  char *base = place_walk(k, w, P->work.p);
   float *sa = R > 1 ? (float *)base : nullptr;
-  base += al(stage_floats * 4);
+  base += al256(stage_floats * 4);
   float *sb = R > 1 ? (float *)base : nullptr;
   for (int c0 = 0; c0 < C; c0 += chunk) {
     const int cc = std::min(chunk, C - c0);
-    int lr = launch_walk_post(k, A, R > 1 ? 3 : 0, tc, sa, sb, c0, cc, walk_grid, stream);
+    int lr = w.q ? launch_qwalk(k, A, w.f81, R > 1, sa, sb, kQLeafU, c0, cc, w.g, stream)
+                 : launch_walk_post(k, A, R > 1 ? 3 : 0, tc, sa, sb, c0, cc, w.grid, stream);
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("walk launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
     if (R == 1) continue;
