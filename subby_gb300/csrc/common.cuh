@@ -131,7 +131,7 @@ int launch_warp(const KParams &p, int A, int grid, int block, size_t smem, cudaS
 int launch_tree(const KParams &p, int A, int store, int grid, int block, size_t smem,
                 cudaStream_t s);
 bool tree_supported(int A);
-// large-alphabet walk + accumulation (k_big.cu)
+// A = 64 walk, large-alphabet accumulation (k_big.cu)
 bool big_supported(int A);
 int big_tile();
 int big_acc_group(int A);
@@ -220,10 +220,11 @@ int launch_acc_cx(const KParams &p, int A, bool pb, const float *sa, const float
 int launch_bt_cx(const KParams &p, int A, const float2 *cbuf, int c_base, int c_count, int row, int grid,
                  cudaStream_t s);
 // reversible large-alphabet gradient (k_grad.cu): X_n += sum_c g_c D~_nc (x) U~_nc
-// from the walk's eigen staging, X (R x A x A) FP64
-int xgram_items(int R, int c_count);
-int launch_xgram(int A, const float *sa, const float *sb, const float *g, int c_base, int c_count, int R, double *X,
-                 int grid, cudaStream_t s);
+// from the eigen staging, X (R x A x A) FP64; then the contraction of every
+// X_n into grad_t (R) and Cg (A x A)
+int launch_xgram(const KParams &p, int A, const float *sa, const float *sb, const float *g, int c_base, int c_count,
+                 double *X, int nsm, cudaStream_t s);
+int launch_xform(const double *X, const double *tab64, int R, int A, double *grad_t, double *Cg, cudaStream_t s);
 // distance gradient from the raw staging: grad_t[n] += sum_c g_c (D s)^T G_n U
 int launch_grad_cx(const KParams &p, int A, const float *sa, const float *sb, const float *gq, const float *g,
                    int c_base, int c_count, double *grad_t, int grid, cudaStream_t s);

@@ -1,6 +1,7 @@
-// Large-alphabet path (A = 16, 20, 32, 64): tree walk + staged accumulation.
+// Large-alphabet path: the A = 64 tree walk, and the accumulation over staged
+// vectors at A = 16, 20, 32, 64 (staged there by k_qwalk and k_proj).
 //
-// Kernel 1, k_walk<A> (walk.cuh): the tree program of k_tree.cu (stored / derived
+// Kernel 1, k_walk<64> (walk.cuh): the tree program of k_tree.cu (stored / derived
 // nodes; subby/oracle/oracle.py:784-924) for a tile of 128 columns per CTA.
 // Thread (c, h) owns column c of the tile and states [32h, 32h + S) of every
 // vector (S = min(A, 32); h < H = ceil(A / 32)), so a length-A vector lives
@@ -624,29 +625,11 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
 #undef ACC
 
 
-// The closed-form F81 walk serves the inside-only and F81-staging modes;
-// eigen staging of an F81 model keeps the general products.
-template <int A, bool TC>
-int walk_launch_tc(const KParams &p, int mode, float *sa, float *sb, int c_base, int c_count, int grid,
-                   cudaStream_t s) {
-  const bool f = !TC && p.f81_model != 0;   // (the tensor-core walk is never F81-specialised)
-  constexpr bool kF = !TC;
-  if (mode == 0)
-    return f ? walk_launch1<A, 0, TC, kF>(p, sa, sb, c_base, c_count, grid, s)
-             : walk_launch1<A, 0, TC, false>(p, sa, sb, c_base, c_count, grid, s);
-  if (mode == 1) return walk_launch1<A, 1, TC, false>(p, sa, sb, c_base, c_count, grid, s);
-  return f ? walk_launch1<A, 2, TC, kF>(p, sa, sb, c_base, c_count, grid, s)
-           : walk_launch1<A, 2, TC, false>(p, sa, sb, c_base, c_count, grid, s);
-}
-
-template <int A>
-int walk_launch(const KParams &p, int mode, bool tc, float *sa, float *sb, int c_base, int c_count, int grid,
-                cudaStream_t s) {
-  if constexpr (A == 64) {
-    // the closed-form F81 walk has no matrix products for the tensor cores
-    if (tc && !(p.f81_model && mode != 1)) return walk_launch_tc<A, true>(p, mode, sa, sb, c_base, c_count, grid, s);
-  }
-  return walk_launch_tc<A, false>(p, mode, sa, sb, c_base, c_count, grid, s);
+template <bool TC>
+int walk_launch(const KParams &p, int mode, float *sa, float *sb, int c_base, int c_count, int grid, cudaStream_t s) {
+  if (mode == 0) return walk_launch1<64, 0, TC, false>(p, sa, sb, c_base, c_count, grid, s);
+  if (mode == 1) return walk_launch1<64, 1, TC, false>(p, sa, sb, c_base, c_count, grid, s);
+  return walk_launch1<64, 2, TC, false>(p, sa, sb, c_base, c_count, grid, s);
 }
 
 template <int A, bool F81, bool TCB, bool PB = false>
@@ -692,13 +675,9 @@ int big_acc_group(int A) {
 
 int launch_walk(const KParams &p, int A, int mode, bool tc, float *sa, float *sb, int c_base, int c_count,
                 int grid, cudaStream_t s) {
-  switch (A) {
-    case 16: return walk_launch<16>(p, mode, false, sa, sb, c_base, c_count, grid, s);
-    case 20: return walk_launch<20>(p, mode, false, sa, sb, c_base, c_count, grid, s);
-    case 32: return walk_launch<32>(p, mode, false, sa, sb, c_base, c_count, grid, s);
-    case 64: return walk_launch<64>(p, mode, tc, sa, sb, c_base, c_count, grid, s);
-    default: return -1;
-  }
+  if (A != 64) return -1;
+  return tc ? walk_launch<true>(p, mode, sa, sb, c_base, c_count, grid, s)
+            : walk_launch<false>(p, mode, sa, sb, c_base, c_count, grid, s);
 }
 
 int launch_acc(const KParams &p, int A, bool f81, bool tc, const float *sa, const float *sb, int c_base,

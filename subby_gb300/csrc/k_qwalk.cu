@@ -443,10 +443,14 @@ __global__ void __launch_bounds__((q_threads<CPL, F81M>()), MINB)
       for (int q = 0; q < CPL; ++q) O.row(q, pr0g, sg);
 #pragma unroll
       for (int q = 0; q < CPL; ++q) {
+        // one sum over the states in their order, as the other walks form it
         float pp = 0.f;
 #pragma unroll
-        for (int i = 0; i < SPL; ++i) pp = fmaf(O.get(q, i), ur.get(q, i), pp);
-        pp = qsum(pp);
+        for (int j = 0; j < A; ++j) {
+          const int i = (A == 20 && j >= 16) ? 4 : (j / 16) * 4 + (j & 3);
+          const int from = ((A == 20 && j >= 16) ? j - 16 : (j % 16) / 4) * 8 + cg;
+          pp = fmaf(__shfl_sync(0xffffffffu, O.get(q, i), from), __shfl_sync(0xffffffffu, ur.get(q, i), from), pp);
+        }
         invP[q] = 1.0f / pp;
         if (cc0 + q < c_count) {
           const size_t col = (size_t)c_base + cc0 + q;

@@ -14,9 +14,12 @@ template <int A, bool TC>
 int walk_post1(const KParams &p, int mode, float *sa, float *sb, int c_base, int c_count, int grid, cudaStream_t s) {
   const bool f = !TC && p.f81_model != 0;
   constexpr bool kF = !TC;
-  if (mode == 0)
+  if constexpr (A == 16 || A == 20 || A == 32) {
+    if (mode == 0) return -1;   // inside-only runs take k_qwalk
+  } else if (mode == 0) {
     return f ? walk_launch1<A, 0, TC, kF>(p, sa, sb, c_base, c_count, grid, s)
              : walk_launch1<A, 0, TC, false>(p, sa, sb, c_base, c_count, grid, s);
+  }
   return f ? walk_launch1<A, 3, TC, kF>(p, sa, sb, c_base, c_count, grid, s)
            : walk_launch1<A, 3, TC, false>(p, sa, sb, c_base, c_count, grid, s);
 }

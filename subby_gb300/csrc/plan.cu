@@ -1272,9 +1272,10 @@ struct WalkPlan {
 };
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-int plan_walk(const subby_plan *P, KParams &k, bool q, bool outside, int chunk, int per_sm, WalkPlan *w) {
+int plan_walk(const subby_plan *P, KParams &k, bool q, bool outside, int chunk, int per_sm, WalkPlan *w,
+              bool closed_form = true) {
   w->outside = outside;
-  w->f81 = P->f81_model != 0;
+  w->f81 = closed_form && P->f81_model != 0;
   w->q = q && qwalk_supported(P->A, w->f81);
   if (w->q) {
     // every internal node stored; inside only: slots reused bottom-up
@@ -1551,8 +1552,9 @@ int run_cx(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_c
 }
 
 // Gradient of reversible large-alphabet plans: the walk's eigen staging
-// (mode 1, unmasked; LogLike from its inside pass) and k_xgram's per-branch
-// X_n = sum_c g_c D~_nc (x) U~_nc accumulated into d_X (R x A x A, FP64).
+// (unmasked; LogLike from its inside pass; at A = 16, 20, 32 the four-lane
+// walk's raw staging and k_proj) and the per-branch column sums of its outer
+// products, accumulated into d_X (R x A x A, FP64).
 int run_big_grad(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, const float *d_g, double *d_X,
                  cudaStream_t stream) {
   const int A = P->A, R = P->R;
@@ -1570,30 +1572,29 @@ int run_big_grad(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, cons
     const size_t even = ((size_t)C + nch - 1) / nch;
     chunk = (int)std::min<size_t>((size_t)C, (even + tile - 1) / tile * tile);
   }
-  const int walk_grid = std::max(1, std::min((chunk + tile - 1) / tile, P->nsm * (H == 2 ? 1 : 2)));
-  const size_t slot_floats = (size_t)walk_grid * k.nslots * tile * A;
-  const size_t slot_ints = (size_t)walk_grid * k.nslots * tile * 2;  // a word per column half
-  const size_t stage_floats = R > 1 ? (size_t)(R - 1) * chunk * A : 0;
-  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  WalkPlan w;
   int rc;
-  if ((rc = P->grow(P->work, al(slot_floats * 4) + al(slot_ints * 4) + 2 * al(stage_floats * 4) + 256, stream)))
-    return rc;
-  char *base = (char *)P->work.p;
-  k.scrV = (float *)base;
-  base += al(slot_floats * 4);
-  k.scrW = (int *)base;
-  base += al(slot_ints * 4);
+  // the gradients are FP64 sums of FP32 products: an F81 model keeps the
+  // general products here
+  if ((rc = plan_walk(P, k, proj_supported(A), R > 1, chunk, H == 2 ? 1 : 2, &w, false))) return rc;
+  const size_t stage_bytes = R > 1 ? al256((size_t)(R - 1) * chunk * A * sizeof(float)) : 0;
+  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * stage_bytes + 256, stream))) return rc;
+  char *base = place_walk(k, w, P->work.p);
   float *sa = (float *)base;
-  base += al(stage_floats * 4);
-  float *sb = (float *)base;
+  float *sb = (float *)(base + stage_bytes);
   for (int c0 = 0; c0 < C; c0 += chunk) {
     const int cc = std::min(chunk, C - c0);
-    int lr = launch_walk(k, A, R > 1 ? 1 : 0, tc, sa, sb, c0, cc, walk_grid, stream);
+    int lr = w.q ? launch_qwalk(k, A, w.f81, R > 1, sa, sb, kQRotate, c0, cc, w.g, stream)
+                 : launch_walk(k, A, R > 1 ? 1 : 0, tc, sa, sb, c0, cc, w.grid, stream);
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("walk launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
     if (R == 1) continue;
-    const int grid = std::max(1, std::min(xgram_items(R, cc), P->nsm * 4));
-    lr = launch_xgram(A, sa, sb, d_g, c0, cc, R, d_X, grid, stream);
+    if (w.q) {
+      lr = launch_proj(k, A, P->hVd.data(), P->hVu.data(), sa, sb, c0, cc, P->nsm, stream);
+      if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("projection launch failed: ") + cudaGetErrorString((cudaError_t)lr));
+      g_launches += 1;
+    }
+    lr = launch_xgram(k, A, sa, sb, d_g, c0, cc, d_X, P->nsm, stream);
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("gradient launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
   }
@@ -2095,39 +2096,30 @@ int subby_plan_grad(subby_plan *P, const int32_t *aln, int C, const float *g, fl
     return SUBBY_OK;
   }
   if (big_supported(A) && g_kernel_sel == 0) {
-    // walk + per-branch X_n (k_grad.cu); the gradients follow on the host in FP64
+    // walk + per-branch sums and their contraction (k_grad.cu), FP64; d_X is
+    // followed by grad_t (R) and Cg (A x A)
     double *d_X = nullptr;
-    const size_t xb = sizeof(double) * (size_t)R * A * A;
-    CU(pool_alloc((void **)&d_X, xb, P->pool, stream));
-    CU(cudaMemsetAsync(d_X, 0, xb, stream));
+    const size_t nx = (size_t)R * A * A, nout = (size_t)R + (size_t)A * A;
+    CU(pool_alloc((void **)&d_X, sizeof(double) * (nx + nout), P->pool, stream));
+    CU(cudaMemsetAsync(d_X, 0, sizeof(double) * (nx + nout), stream));
     rc = run_big_grad(P, d_aln, C, logL ? d_ll : nullptr, d_g, d_X, stream);
-    std::vector<double> X((size_t)R * A * A);
+    if (rc == 0 && R > 1) {
+      const int lr = launch_xform(d_X, P->d_tab64, R, A, d_X + nx, d_X + nx + R, stream);
+      if (lr != 0) rc = fail(SUBBY_ERR_CUDA, std::string("gradient launch failed: ") + cudaGetErrorString((cudaError_t)lr));
+      else g_launches += 1;
+    }
+    std::vector<double> res(nout, 0.0);
     cudaError_t e = cudaSuccess;
-    if (rc == 0) e = cudaMemcpyAsync(X.data(), d_X, xb, cudaMemcpyDeviceToHost, stream);
+    if (rc == 0) e = cudaMemcpyAsync(res.data(), d_X + nx, sizeof(double) * nout, cudaMemcpyDeviceToHost, stream);
     if (rc == 0 && e == cudaSuccess && logL && !dev)
       e = cudaMemcpyAsync(logL, d_ll, (size_t)C * 4, cudaMemcpyDeviceToHost, stream);
     cudaFreeAsync(d_X, stream);
     cudaError_t e2 = cudaStreamSynchronize(stream);
     if (rc) return rc;
     if (e != cudaSuccess || e2 != cudaSuccess) return cuda_fail(e != cudaSuccess ? e : e2, "gradient readback");
-    // d/dt_n = sum_k mu_k e^{mu_k t_n} X_n[k][k];  Cg = sum_n J_n o X_n
-    // (J with the 1e-8 degeneracy rule, subby/oracle/oracle.py:931-959)
-    std::vector<double> Cg((size_t)A * A, 0.0), E(A);
+    std::copy(res.begin(), res.begin() + R, dldt);
     dldt[0] = 0.0;
-    for (int n = 1; n < R; ++n) {
-      const double tn = P->t[n];
-      const double *Xn = X.data() + (size_t)n * A * A;
-      for (int k2 = 0; k2 < A; ++k2) E[k2] = std::exp(P->mu[k2] * tn);
-      double gd = 0.0;
-      for (int k2 = 0; k2 < A; ++k2) gd += P->mu[k2] * E[k2] * Xn[k2 * A + k2];
-      dldt[n] = gd;
-      for (int k2 = 0; k2 < A; ++k2)
-        for (int l = 0; l < A; ++l) {
-          const double d = P->mu[k2] - P->mu[l];
-          const double J = std::fabs(d) < 1e-8 ? tn * E[k2] : (E[k2] - E[l]) / d;
-          Cg[k2 * A + l] += J * Xn[k2 * A + l];
-        }
-    }
+    const double *Cg = res.data() + R;
     const std::vector<double> &V = P->V;
     std::vector<double> T((size_t)A * A, 0.0);
     for (int k2 = 0; k2 < A; ++k2)

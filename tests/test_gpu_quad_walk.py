@@ -88,3 +88,24 @@ def test_closed_form(A, C):
     aln, t, m, md, ot = _case(A, "f81", "random", C, A + C)
     _check(aln, t, m, md, ot, np.arange(C), True, "auto")
     _check(aln, t, m, md, ot, np.arange(C), False, None)
+
+
+@pytest.mark.parametrize("A", [16, 20, 32])
+@pytest.mark.parametrize("C", [1, 37, 4097])
+def test_gradient(A, C):
+    """Branch-length gradient with weights: fewer branches than a CTA's group
+    of them and one left over, column blocks of 4096 and a remainder."""
+    for tree in ("pair", "random", "caterpillar"):
+        aln, t, m, md, ot = _case(A, "reversible", tree, C, 3 * A + C)
+        g = np.random.default_rng(C).integers(1, 5, size=C).astype(np.float64)
+        plan = sg.Plan(t, m)
+        ll, dt, dS = plan.grad(aln, g)
+        plan.close()
+        assert_loglike(ll, oracle.LogLike(aln, ot, md))
+        ref = oracle.loglike_distance_grad(aln, ot, md, g)
+        assert np.abs(dt - ref).max() <= 1e-4 * np.abs(ref).max()
+        # V^T dS V = sum_n J_n o X_n and J_n[k][k] = t_n e^{mu_k t_n}, so its
+        # mu-weighted trace is sum_n t_n d/dt_n
+        V, tn = np.asarray(m.eigenvectors), np.asarray(t.distanceToParent)
+        trace = (np.diag(V.T @ dS @ V) * np.asarray(m.eigenvalues)).sum()
+        assert abs(trace - (dt * tn).sum()) <= 1e-9 * np.abs(dt * tn).sum()
