@@ -219,6 +219,29 @@ int launch_acc_cx(const KParams &p, int A, bool pb, const float *sa, const float
                   int n_lo, int n_hi, float2 *cbuf, int grid, cudaStream_t s);
 int launch_bt_cx(const KParams &p, int A, const float2 *cbuf, int c_base, int c_count, int row, int grid,
                  cudaStream_t s);
+// irreversible counts at A = 16, 20, 32 for eigensystems in conjugate pairs
+// (k_accx.cu): the units' tables on the device (U units, padded to an even
+// UP, the first `pairs` of them conjugate pairs, then reals; G columns per
+// block) and the real-form projection matrices on the host
+struct CxUnits {
+  int U, UP, pairs, G;
+  const float *J;        // R x UP x UP x (J_kl, J_kl')
+  const float *leafU;    // (A + 1) x A: U~ of a token, real form
+  const float2 *V;       // A x UP: weight x V of the representatives
+  const float2 *Vi;      // UP x 2 x A: Vinv of the representative, of its partner
+  const float *rate;     // A x A
+};
+struct CxHost {
+  const float *d, *u;    // A x A [state][output]
+  const uint8_t *slot;   // output -> row of the projected block
+};
+bool accx_supported(int A);
+// floats between the rows of a projected block of G columns: rows of units
+// four apart start 8 banks apart
+__host__ __device__ constexpr int accx_stride(int G) { return G + 2; }
+int accx_group(int A, int UP);
+int launch_accx(const KParams &p, int A, const CxUnits &cu, const CxHost &h, const float *sa, const float *sb,
+                float *pa, float *pb, int c_base, int c_count, int nsm, cudaStream_t s);
 // reversible large-alphabet gradient (k_grad.cu): X_n += sum_c g_c D~_nc (x) U~_nc
 // from the eigen staging, X (R x A x A) FP64; then the contraction of every
 // X_n into grad_t (R) and Cg (A x A)

@@ -270,6 +270,14 @@ struct subby_plan {
   int ngroups = 1;
   std::vector<int> grp_off;
   int *d_grp_br = nullptr;
+  // irreversible plans whose eigensystem pairs up (k_accx): the units, the
+  // device tables (one buffer: J, then per formula leafU, V, Vinv, rate) and
+  // the real-form projections, for the reference's formula and the exact one
+  CxUnits cxu{};
+  float *d_cxu = nullptr;
+  std::vector<float> cxd[2], cxup[2];
+  std::vector<uint8_t> cx_slot;
+  size_t cx_stride = 0;    // floats of one formula's tables
   float *d_gq = nullptr;   // complex-system plans: dM_n/dt = Re V diag(mu e^{mu t_n}) V^-1 (R x A x A)
   TableOffsets off{};
   float *d_tab = nullptr;
@@ -369,6 +377,49 @@ struct IrrevInput {
   const double *mu, *V, *Vi;
   int per_row;
 };
+
+// The units of an irreversible eigensystem: representatives in order
+// (conjugate pairs, then reals), partner[u] the conjugate's index or -1.
+// False when the values or vectors do not pair up to 1e-9.
+bool cx_pair_up(const IrrevInput &ir, int A, std::vector<int> &rep, std::vector<int> &partner) {
+  using cd = std::complex<double>;
+  auto mu = [&](int k) { return cd(ir.mu[2 * k], ir.mu[2 * k + 1]); };
+  auto V = [&](int i, int k) { return cd(ir.V[2 * (i * A + k)], ir.V[2 * (i * A + k) + 1]); };
+  auto Vi = [&](int k, int j) { return cd(ir.Vi[2 * (k * A + j)], ir.Vi[2 * (k * A + j) + 1]); };
+  // does index m hold the conjugate of index k (m = k: is k real)?
+  auto conj_of = [&](int k, int m) {
+    if (std::abs(mu(m) - std::conj(mu(k))) > 1e-9 * std::max(1.0, std::abs(mu(k)))) return false;
+    double vs = 0.0, is = 0.0, vd = 0.0, id = 0.0;
+    for (int a = 0; a < A; ++a) {
+      vs = std::max(vs, std::abs(V(a, k)));
+      is = std::max(is, std::abs(Vi(k, a)));
+      vd = std::max(vd, std::abs(V(a, m) - std::conj(V(a, k))));
+      id = std::max(id, std::abs(Vi(m, a) - std::conj(Vi(k, a))));
+    }
+    return vd <= 1e-9 * vs && id <= 1e-9 * is;   // (false for NaN)
+  };
+  std::vector<char> used(A, 0);
+  std::vector<int> reals;
+  for (int k = 0; k < A; ++k) {
+    if (used[k]) continue;
+    used[k] = 1;
+    if (conj_of(k, k)) {
+      reals.push_back(k);
+      continue;
+    }
+    int m = k + 1;
+    while (m < A && (used[m] || !conj_of(k, m))) ++m;
+    if (m == A) return false;
+    used[m] = 1;
+    rep.push_back(k);
+    partner.push_back(m);
+  }
+  for (int k : reals) {
+    rep.push_back(k);
+    partner.push_back(-1);
+  }
+  return true;
+}
 
 int plan_create(const int32_t *parent, const double *dist, const double *evals, const double *evecs,
                 const double *pi, int R, int A, subby_plan **out, const IrrevInput *ir) {
@@ -780,6 +831,81 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
           put64(3, e, V_of(n, et));
         }
     }
+    std::vector<int> rep_u, partner;
+    if (!ir->per_row && accx_supported(A) && R > 1 && cx_pair_up(*ir, A, rep_u, partner)) {
+      CxUnits &cu = P->cxu;
+      cu.U = (int)rep_u.size();
+      cu.UP = (cu.U + 1) & ~1;
+      cu.pairs = (int)std::count_if(partner.begin(), partner.end(), [](int m) { return m >= 0; });
+      cu.G = accx_group(A, cu.UP);
+      const int U = cu.U, UP = cu.UP;
+      // J_kl, J_kl' of the representatives; zero for padding and for the
+      // missing partner of a real
+      const size_t nj = (size_t)R * UP * UP * 4;
+      const size_t n_leaf = (size_t)(A + 1) * A, n_v = 2 * (size_t)A * UP, n_vi = 4 * (size_t)UP * A, n_r = AA;
+      P->cx_stride = n_leaf + n_v + n_vi + n_r;
+      std::vector<float> h(nj + 2 * P->cx_stride, 0.f);
+      for (int n = 0; n < R; ++n)
+        for (int k = 0; k < U; ++k)
+          for (int l = 0; l < U; ++l) {
+            float *q = h.data() + (((size_t)n * UP + k) * UP + l) * 4;
+            const float2 *Jn = hcx.data() + (size_t)n * AA + (size_t)rep_u[k] * A;
+            q[0] = Jn[rep_u[l]].x, q[1] = Jn[rep_u[l]].y;
+            if (partner[l] >= 0) q[2] = Jn[partner[l]].x, q[3] = Jn[partner[l]].y;
+          }
+      for (int x = 0; x < 2; ++x) {
+        // the system of the formula: (V, Vinv), or (Vinv^T, V^T) for the exact one
+        auto Vx = [&](int i, int k) { return x ? Vi_of(0, (size_t)k * A + i) : V_of(0, (size_t)i * A + k); };
+        auto Vix = [&](int k, int j) { return x ? V_of(0, (size_t)j * A + k) : Vi_of(0, (size_t)k * A + j); };
+        P->cxd[x].assign(AA, 0.f);
+        P->cxup[x].assign(AA, 0.f);
+        P->cx_slot.clear();
+        std::vector<double> up(AA);
+        int col = 0;
+        auto put = [&](int u, bool imag) {
+          for (int a = 0; a < A; ++a) {
+            const cd dz = Vix(rep_u[u], a), uz = Vx(a, rep_u[u]);
+            P->cxd[x][(size_t)a * A + col] = (float)(imag ? dz.imag() : dz.real());
+            up[(size_t)a * A + col] = imag ? uz.imag() : uz.real();
+            P->cxup[x][(size_t)a * A + col] = (float)up[(size_t)a * A + col];
+          }
+          P->cx_slot.push_back((uint8_t)(2 * u + (imag ? 1 : 0)));
+          ++col;
+        };
+        for (int u = 0; u < U; ++u) {
+          put(u, false);
+          if (partner[u] >= 0) put(u, true);
+        }
+        float *leafU = h.data() + nj + x * P->cx_stride, *hV = leafU + n_leaf, *hVi = hV + n_v, *hR = hVi + n_vi;
+        for (int o2 = 0; o2 < A; ++o2) {
+          double sum = 0.0;
+          for (int b = 0; b < A; ++b) {
+            leafU[(size_t)b * A + o2] = P->cxup[x][(size_t)b * A + o2];
+            sum += up[(size_t)b * A + o2];
+          }
+          leafU[AA + o2] = (float)sum;
+        }
+        for (int u = 0; u < U; ++u)
+          for (int a = 0; a < A; ++a) {
+            const cd v = Vx(a, rep_u[u]) * (partner[u] >= 0 ? 2.0 : 1.0), w1 = Vix(rep_u[u], a);
+            hV[2 * ((size_t)a * UP + u)] = (float)v.real();
+            hV[2 * ((size_t)a * UP + u) + 1] = (float)v.imag();
+            hVi[2 * ((size_t)2 * u * A + a)] = (float)w1.real();
+            hVi[2 * ((size_t)2 * u * A + a) + 1] = (float)w1.imag();
+            if (partner[u] >= 0) {
+              const cd w2 = Vix(partner[u], a);
+              hVi[2 * ((size_t)(2 * u + 1) * A + a)] = (float)w2.real();
+              hVi[2 * ((size_t)(2 * u + 1) * A + a) + 1] = (float)w2.imag();
+            }
+          }
+        const float2 *R0 = hcx.data() + (size_t)(R + 2) * AA;   // rate matrix of group 0
+        for (size_t e2 = 0; e2 < AA; ++e2) hR[e2] = R0[e2].x;
+      }
+      e = pool_alloc((void **)&P->d_cxu, h.size() * sizeof(float), P->pool, qs);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(P->d_cxu, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice, qs);
+      if (e != cudaSuccess) return cleanup(cuda_fail(e, "irreversible unit tables"));
+    }
     e = cudaMemcpyAsync(P->d_tab + o.MT, hMT.data(), hMT.size() * sizeof(float), cudaMemcpyHostToDevice, qs);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(P->d_tab + o.MN, hMN.data(), hMN.size() * sizeof(float), cudaMemcpyHostToDevice, qs);
@@ -899,7 +1025,7 @@ int subby_plan_destroy(subby_plan *P) {
   if (s && P->used) cudaStreamWaitEvent(s, P->last_use, 0);
   if (P->s_in) cudaStreamSynchronize(P->s_in);
   if (P->s_out) cudaStreamSynchronize(P->s_out);
-  void *bufs[] = {P->d_tab, P->d_tab64, P->d_steps, P->d_slots, P->d_prog, P->d_prog_w, P->d_prog_s, P->d_leaf, P->d_tab16, P->d_err,
+  void *bufs[] = {P->d_tab, P->d_tab64, P->d_steps, P->d_slots, P->d_prog, P->d_prog_w, P->d_prog_s, P->d_leaf, P->d_cxu, P->d_tab16, P->d_err,
                   P->d_cx, P->d_grp_br, P->d_gq};
   for (void *b : bufs)
     if (b) cudaFreeAsync(b, s);
@@ -1480,13 +1606,16 @@ int run_cx(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_c
   k.cx_exact = P->rows || (mode & kModeIrrevExact) != 0;
   k.npost = nullptr;
   k.npost_node = -1;
+  // conjugate-paired systems at A = 16, 20, 32: k_accx
+  const bool units = counts && !pb && P->d_cxu && P->cxu.G > 0;
   const bool bt64 = cx_bt64(A) && !P->rows;   // per-branch reversible systems are well conditioned
   const bool tc = (A == 64) && P->d_tab16 && (g_kernel_sel == 0 || g_kernel_sel == 5);
   const int tile = big_tile();
   const int H = (A + 31) / 32;
   int chunk = C;
   if (counts) {
-    const size_t per_col = (size_t)2 * (R - 1) * A * sizeof(float);
+    // (with the projected vectors beside the raw ones for k_accx)
+    const size_t per_col = (size_t)2 * (R - 1) * (A + (units ? 2 * P->cxu.UP : 0)) * sizeof(float);
     size_t cmax = std::max<size_t>(tile, kStageBudget / per_col);
     cmax = cmax / tile * tile;
     const size_t nch = ((size_t)C + cmax - 1) / cmax;
@@ -1498,8 +1627,10 @@ int run_cx(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_c
   int rc;
   if ((rc = plan_walk(P, k, true, counts, chunk, per_sm, &w))) return rc;
   const size_t stage_floats = counts ? (size_t)(R - 1) * chunk * A : 0;
+  const size_t unit_blocks = units ? ((size_t)chunk + P->cxu.G - 1) / P->cxu.G : 0;
+  const size_t proj_bytes = al256((size_t)(R - 1) * unit_blocks * 2 * P->cxu.UP * accx_stride(P->cxu.G) * sizeof(float));
   const size_t cbuf_bytes = (counts && bt64) ? (size_t)chunk * A * A * sizeof(float2) : 0;
-  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + al256(cbuf_bytes) + 256,
+  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + al256(cbuf_bytes) + 2 * proj_bytes + 256,
                     stream)))
     return rc;
   char *base = place_walk(k, w, P->work.p);
@@ -1508,14 +1639,33 @@ int run_cx(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_c
   float *sb = counts ? (float *)base : nullptr;
   base += al256(stage_floats * 4);
   float2 *cbuf = cbuf_bytes ? (float2 *)base : nullptr;
+  CxUnits cu = P->cxu;
+  const int xi = k.cx_exact ? 1 : 0;
+  if (units) {
+    const int UP = cu.UP;
+    cu.J = P->d_cxu;
+    cu.leafU = P->d_cxu + (size_t)R * UP * UP * 4 + xi * P->cx_stride;
+    cu.V = (const float2 *)(cu.leafU + (size_t)(A + 1) * A);
+    cu.Vi = cu.V + (size_t)A * UP;
+    cu.rate = (const float *)(cu.Vi + 2 * (size_t)UP * A);
+  }
   const int G = cx_columns_per_cta(A);
   for (int c0 = 0; c0 < C; c0 += chunk) {
     const int cc = std::min(chunk, C - c0);
-    int lr = w.q ? launch_qwalk(k, A, w.f81, counts, sa, sb, kQLeafU, c0, cc, w.g, stream)
+    int lr = w.q ? launch_qwalk(k, A, w.f81, counts, sa, sb, units ? kQRotate : kQLeafU, c0, cc, w.g, stream)
                  : launch_walk_post(k, A, counts ? 3 : 0, tc, sa, sb, c0, cc, w.grid, stream);
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("walk launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
     if (!counts) continue;
+    if (units) {
+      float *pa = (float *)base, *pbuf = (float *)(base + proj_bytes);
+      const CxHost h{P->cxd[xi].data(), P->cxup[xi].data(), P->cx_slot.data()};
+      lr = launch_accx(k, A, cu, h, sa, sb, pa, pbuf, c0, cc, P->nsm, stream);
+      if (lr != 0)
+        return fail(SUBBY_ERR_CUDA, std::string("accumulate launch failed: ") + cudaGetErrorString((cudaError_t)lr));
+      g_launches += 2;
+      continue;
+    }
     const long long groups = (cc + G - 1) / G;
     const int grid = (int)std::max<long long>(1, std::min<long long>(groups, (long long)P->nsm * 2));
     if (!bt64) {
