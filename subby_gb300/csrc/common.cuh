@@ -182,6 +182,10 @@ int launch_acc(const KParams &p, int A, bool f81, bool tc, const float *sa, cons
                int c_count, int grid, cudaStream_t s);
 int launch_tree4(const KParams &p, bool f81, int mask_mode, int grid, int block, size_t smem,
                  cudaStream_t s);
+// A = 4 inside pass only (k_inside4.cu): LogLike / RootProb
+// (per: columns per thread, 1 or 2)
+size_t inside4_smem(int R, int nsteps, int nslots, int block, int per);
+int launch_inside4(const KParams &p, int per, int grid, int block, size_t smem, cudaStream_t s);
 // Packed queue of (job, column range) work items of the A = 4 serving
 // kernel (k_tree4_packed): jobs[j] are the tree-kernel parameters of job j,
 // items are (job, first column, end column) of a run of whole tiles of

@@ -3,6 +3,8 @@
 // dispatch.  See include/subby_gb300.h for the contract.
 #include <cuda_runtime.h>
 
+#include <limits.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -254,6 +256,10 @@ struct subby_plan {
   std::vector<int4> prog, prog_w, prog_s;
   int prog_steps = 0, prog_slots = 0, prog_w_steps = 0, prog_w_slots = 0, prog_s_slots = 0;
   int4 *d_prog = nullptr, *d_prog_w = nullptr, *d_prog_s = nullptr;
+  // A = 4, inside only (k_inside4): one int4 per internal node
+  std::vector<int4> prog_i;
+  int prog_i_slots = 0;
+  int4 *d_prog_i = nullptr;
   uint8_t *d_leaf = nullptr;          // (R,) 1 for leaves
   std::vector<float> hVd, hVu;        // FP32 projection matrices (kernel parameters of k_proj)
   std::vector<double> V, mu, pi, t;   // FP64 model and branch lengths (host)
@@ -559,6 +565,53 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
     }
   }
 
+  if (A == 4 && R > 1) {
+    // need[v]: slots that the subtree of v holds at once when the child with
+    // the larger need goes first
+    std::vector<int> need(R, 0);
+    for (int v : order) {
+      const int l = left[v], r = right[v];
+      const bool li = left[l] >= 0, ri = left[r] >= 0;
+      const int a = std::max(need[l], need[r]), b = std::min(need[l], need[r]);
+      need[v] = (li && ri) ? std::max(a, b + 1) : a;
+    }
+    P->prog_i_slots = need[0];
+    std::vector<int> slot_of(R, -1);
+    std::vector<std::pair<int, int>> st;   // node, state (0: enter, 1: first child done, 2: both)
+    int sp = 0, last = -1;
+    st.push_back({0, 0});
+    while (!st.empty()) {
+      const int v = st.back().first;
+      const int l = left[v], r = right[v];
+      const bool li = left[l] >= 0, ri = left[r] >= 0;
+      const bool right_first = ri && (!li || need[r] > need[l]);
+      const int first = right_first ? r : l, second = right_first ? l : r;
+      int &state = st.back().second;
+      if (state == 0) {
+        state = 1;
+        if (left[first] >= 0) {
+          st.push_back({first, 0});
+          continue;
+        }
+      }
+      if (state == 1) {
+        state = 2;
+        if (left[second] >= 0) {
+          // the first child's vector waits in a slot
+          slot_of[first] = sp++;
+          P->prog_i.back().w = slot_of[first];
+          st.push_back({second, 0});
+          continue;
+        }
+      }
+      auto ref = [&](int c) { return left[c] < 0 ? c : c == last ? INT_MIN : ~slot_of[c]; };
+      P->prog_i.push_back(make_int4(v, ref(l), ref(r), -1));
+      if (slot_of[first] >= 0) --sp;
+      last = v;
+      st.pop_back();
+    }
+  }
+
   // ---- FP64 host tables
   P->t.assign(dist, dist + R);
   P->V.assign(evecs, evecs + (size_t)A * A);
@@ -707,6 +760,12 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(P->d_prog_s, P->prog_s.data(), sizeof(int4) * P->prog_s.size(), cudaMemcpyHostToDevice,
                           qs);
+    if (e == cudaSuccess && !P->prog_i.empty()) {
+      e = pool_alloc((void **)&P->d_prog_i, sizeof(int4) * P->prog_i.size(), P->pool, qs);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(P->d_prog_i, P->prog_i.data(), sizeof(int4) * P->prog_i.size(), cudaMemcpyHostToDevice,
+                            qs);
+    }
     std::vector<uint8_t> leaf((size_t)R);
     for (int n = 0; n < R; ++n) leaf[n] = left[n] < 0;
     if (e == cudaSuccess) e = pool_alloc((void **)&P->d_leaf, leaf.size(), P->pool, qs);
@@ -1025,7 +1084,7 @@ int subby_plan_destroy(subby_plan *P) {
   if (s && P->used) cudaStreamWaitEvent(s, P->last_use, 0);
   if (P->s_in) cudaStreamSynchronize(P->s_in);
   if (P->s_out) cudaStreamSynchronize(P->s_out);
-  void *bufs[] = {P->d_tab, P->d_tab64, P->d_steps, P->d_slots, P->d_prog, P->d_prog_w, P->d_prog_s, P->d_leaf, P->d_cxu, P->d_tab16, P->d_err,
+  void *bufs[] = {P->d_tab, P->d_tab64, P->d_steps, P->d_slots, P->d_prog, P->d_prog_w, P->d_prog_s, P->d_prog_i, P->d_leaf, P->d_cxu, P->d_tab16, P->d_err,
                   P->d_cx, P->d_grp_br, P->d_gq};
   for (void *b : bufs)
     if (b) cudaFreeAsync(b, s);
@@ -1137,6 +1196,7 @@ struct Launch {
   KParams kp{};
   int kernel = 0;        // 0 small (thread/column), 1 warp/column, 2 tree program
   bool global_slots = false;
+  int columns = 1;       // per thread (k_inside4)
   int store = 0;         // k_tree slot storage: 0 shared, 1 global, 2 tensor memory
   bool small = true;
   int grid = 1, block = 128;
@@ -1332,6 +1392,37 @@ int plan_tree4(subby_plan *P, int mode, int C, Launch &L) {
   k.prog = P->d_prog;
   k.nsteps = P->prog_steps;
   k.nslots = P->prog_slots;
+  return 0;
+}
+
+// A = 4 without an outside pass (k_inside4).  Returns 1 when it does not
+// apply: other modes, or tables too large for shared memory beside the slots.
+int plan_inside4(subby_plan *P, int mode, int C, Launch &L) {
+  if (P->A != 4 || g_kernel_sel != 0 || (mode & ~(kModeLogLike | kModeRootProb | kModeBT64)) != 0) return 1;
+  int maxsm = 0;
+  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, P->device);
+  KParams &k = L.kp;
+  k.prog = P->d_prog_i;
+  k.nsteps = (int)P->prog_i.size();
+  k.nslots = P->prog_i_slots;
+  // Few columns: small CTAs, one per SM first.  Two columns per thread when
+  // one each would take a second wave (1024 threads per SM; R = 199: 200003
+  // columns 103 us with one, 71 us with two; 116736 columns, within a wave,
+  // 48 against 56 us).
+  L.block = 256;
+  while (L.block > 64 && C < P->nsm * L.block) L.block /= 2;
+  int &per = L.columns;
+  per = C > 1024 * P->nsm ? 2 : 1;
+  auto bytes = [&]() { return inside4_smem(P->R, k.nsteps, k.nslots, L.block, per); };
+  if (bytes() > (size_t)maxsm) per = 1;
+  while (bytes() > (size_t)maxsm && L.block > 64) L.block /= 2;
+  L.smem = bytes();
+  if (L.smem > (size_t)maxsm) return 1;
+  const int per_sm = std::max(1, std::min((per == 2 ? 768 : 1024) / L.block, (int)(((size_t)maxsm + 1024) / (L.smem + 1024))));
+  L.kernel = 4;
+  L.small = false;
+  L.grid = std::max(1, std::min((C + L.block * per - 1) / (L.block * per), P->nsm * per_sm));
+  L.nworkers = L.grid * L.block;
   return 0;
 }
 
@@ -1847,8 +1938,10 @@ int run_common(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float 
   const bool tree = tree_supported(P->A) && !(mode & kModeGrad) && g_kernel_sel != 1;
   const bool small = small_supported(P->A);
   int rc;
-  bool tree4 = false;
-  if (tree && (rc = plan_tree4(P, mode, C, L)) == 0) {
+  bool tree4 = false, inside4 = false;
+  if (tree && plan_inside4(P, mode, C, L) == 0) {
+    inside4 = true;
+  } else if (tree && (rc = plan_tree4(P, mode, C, L = Launch())) == 0) {
     tree4 = true;
   } else {
     L = Launch();
@@ -1887,7 +1980,8 @@ int run_common(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float 
   k.scrV = (float *)P->work.p;
   k.scrW = (int *)((char *)P->work.p + vb_al);
   if (grid_out) *grid_out = L.grid;
-  int lr = tree4 ? launch_tree4(k, (mode & kModeF81) != 0, mask_mode, L.grid, L.block, L.smem, stream)
+  int lr = inside4 ? launch_inside4(k, L.columns, L.grid, L.block, L.smem, stream)
+           : tree4 ? launch_tree4(k, (mode & kModeF81) != 0, mask_mode, L.grid, L.block, L.smem, stream)
            : tree ? launch_tree(k, P->A, L.store, L.grid, L.block, L.smem, stream)
            : small ? launch_small(k, P->A, L.grid, L.block, L.smem, stream)
                    : launch_warp(k, P->A, L.grid, L.block, L.smem, stream);
