@@ -6,6 +6,8 @@
 namespace subby {
 namespace {
 
+// what an outside pass writes (k_tree4.cu, k_pass4.cu)
+constexpr int kOutSum = 0, kOutBranch = 1, kOutPost = 2;
 constexpr double kLn2q = 0.69314718055994530942;
 
 struct F4 {

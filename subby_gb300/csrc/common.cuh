@@ -112,6 +112,8 @@ struct KParams {
   int npost_node;
   // (R,) 1 for leaves
   const uint8_t *leaf;
+  // k_pass4_packed: per step, the step of the internal child that waits on the stack
+  const int *prog_other;
   // branch joint posteriors (k_tree4, A = 4): (R, 4, 4, C) or the (4, 4, C)
   // of node npost_node
   float *bpost;
@@ -186,14 +188,22 @@ int launch_tree4(const KParams &p, bool f81, int mask_mode, int grid, int block,
 // (per: columns per thread, 1 or 2)
 size_t inside4_smem(int R, int nsteps, int nslots, int block, int per);
 int launch_inside4(const KParams &p, int per, int grid, int block, size_t smem, cudaStream_t s);
+// A = 4 inside + outside with the nodes' vectors in global memory
+// (k_pass4.cu): counts, or (post) the posteriors of p.npost / p.bpost
+int pass4_steps();   // longest program
+size_t pass4_smem(int R, int nslots, int block, int per, bool f81, bool post);
+int launch_pass4(const KParams &p, const int4 *prog, const int *other, const float *vd, const float *vu, const float *pi, bool f81, int mask_mode, bool post,
+                 int per, int grid, int block, size_t smem, cudaStream_t s);
 // Packed queue of (job, column range) work items of the A = 4 serving
-// kernel (k_tree4_packed): jobs[j] are the tree-kernel parameters of job j,
-// items are (job, first column, end column) of a run of whole tiles of
-// blockDim.x columns (how many tiles an item spans is the work-item shape
-// the serving autotuner picks).  CTAs claim items with an atomic counter; an
-// item at or past *published is waited for (at most wait_polls polls) until
-// *closed is set, and a wait that gives up increments *err and ends the CTA.
-struct T4Queue {
+// kernel (k_pass4_packed): jobs[j] are the parameters of job j, items are
+// (job, first column, end column) of a run of whole tiles of kPackBlock
+// columns (how many tiles an item spans is the work-item shape the serving
+// autotuner picks).  CTAs claim items with an atomic counter; an item at or
+// past *published is waited for (at most wait_polls polls) until *closed is
+// set, and a wait that gives up increments *err and ends the CTA.  scrV,
+// scrW: the CTAs' node slots, max_steps x kPackBlock each.
+constexpr int kPackBlock = 256;
+struct P4Queue {
   const KParams *jobs;
   const int4 *items;
   int *head;
@@ -201,9 +211,12 @@ struct T4Queue {
   const int *closed;
   int wait_polls;
   int *err;
+  int max_steps;
+  float4 *scrV;
+  int *scrW;
 };
-int launch_tree4_packed(const T4Queue &q, bool f81, int mask_mode, int grid, int block, size_t smem,
-                        cudaStream_t s);
+size_t pass4_packed_smem(int R, int nsteps, int nslots, bool f81);
+int launch_pass4_packed(const P4Queue &q, bool f81, int mask_mode, int grid, size_t smem, cudaStream_t s);
 // Row-strided copy by the SMs (k_token.cu): rows x width bytes (width a
 // multiple of 4), e.g. device results into pinned host memory.
 int launch_copy_rows(void *dst, size_t dpitch, const void *src, size_t spitch, size_t width, int rows,
@@ -255,8 +268,6 @@ int launch_xform(const double *X, const double *tab64, int R, int A, double *gra
 // distance gradient from the raw staging: grad_t[n] += sum_c g_c (D s)^T G_n U
 int launch_grad_cx(const KParams &p, int A, const float *sa, const float *sb, const float *gq, const float *g,
                    int c_base, int c_count, double *grad_t, int grid, cudaStream_t s);
-// A = 4 posteriors (npost / bpost) from the tree-program kernel
-int launch_tree4_post(const KParams &p, int grid, int block, size_t smem, cudaStream_t s);
 // A = 64 F81 accumulation on the tensor cores (k_acctc.cu); groups of 8 columns
 int launch_acc_f81_tc(const KParams &p, const float *sa, const float *sb, const float2 *sc, int c_base,
                       int c_count, int grid, cudaStream_t s);

@@ -60,11 +60,7 @@ struct N4 {
 //   stab[3] K    R x 5 x 20 (eigen: K_n[code][k][l] = J_n[k][l] Ut[code][l], rows padded)
 //   stab[4] LV   5 x 4 (observation rows), followed by piL[5] (pi . L(code))
 // OUT: kOutSum, the counts summed over branches; kOutBranch, per-branch
-// counts (R, 4, 4, C) written branch by branch; kOutPost, node posteriors
-// (npost) and / or branch joint posteriors (bpost) of every non-root node
-// (InsideOutside.node_posterior / branch_posterior, subby/oracle/oracle.py:
-// 1755-1905), the root's row from RootProb.
-constexpr int kOutSum = 0, kOutBranch = 1, kOutPost = 2;
+// counts (R, 4, 4, C) written branch by branch.
 
 // P's tables and tree program into shared memory, and the observation rows
 // L(code) (all threads; the caller synchronises before t4_piL).
@@ -239,8 +235,7 @@ __device__ __forceinline__ void t4_cols(const KParams &P, float *sm, const uint3
     P.rootp[(size_t)2 * C + col] = q.b.x;
     P.rootp[(size_t)3 * C + col] = q.b.y;
   }
-  if (!(P.mode & kModeCounts) && OUT != kOutPost) return;
-  if (OUT == kOutPost && (nst == 0 || P.npost_node == 0)) return;
+  if (!(P.mode & kModeCounts)) return;
   if (nst == 0) {
     if (valid)
       for (int i = 0; i < 16; ++i) P.counts[(size_t)i * C + col] = 0.f;
@@ -268,41 +263,6 @@ __device__ __forceinline__ void t4_cols(const KParams &P, float *sm, const uint3
   auto branch = [&](int n, const F4 &D, const F4 &U, int code, int eDU, int active) {
     float s = invP * __int_as_float((max(-127, min(127, eDU - eRoot)) + 127) << 23);
     if (MASK != kMaskNone) s = active ? s : 0.f;
-    if constexpr (OUT == kOutPost) {
-      // y = D^T M_n; node posterior y o U / Z, branch joint D_i M_n[i][j] U_j / Z
-      (void)s;
-      if (P.npost_node >= 0 && n != P.npost_node) return;
-      const float *Mn = MT + n * 20;
-      const F4 p = mul4(vecmat4(Mn, D), U);
-      const float z = sum4(p);
-      const float inv = z > 0.f ? 1.0f / z : 1.0f;
-      if (!valid) return;
-      const size_t row = P.npost_node < 0 ? (size_t)n : 0;
-      if (P.npost) {
-        // streamed stores: the posteriors are written once and not re-read here
-        float *o = P.npost + row * 4 * C + col;
-        __stcs(o, p.a.x * inv);
-        __stcs(o + C, p.a.y * inv);
-        __stcs(o + (size_t)2 * C, p.b.x * inv);
-        __stcs(o + (size_t)3 * C, p.b.y * inv);
-      }
-      if (P.bpost) {
-        float *o = P.bpost + row * 16 * C + col;
-        const F4 ui = scale4(U, inv);
-        const float dk[4] = {D.a.x, D.a.y, D.b.x, D.b.y};
-#pragma unroll
-        for (int i2 = 0; i2 < 4; ++i2) {
-          // row i of M_n is column i of the MT rows: M_n[i][j] = MT[n][j][i]
-          const F4 mi = F4{make_float2(Mn[i2], Mn[4 + i2]), make_float2(Mn[8 + i2], Mn[12 + i2])};
-          const F4 r = scale4(mul4(mi, ui), dk[i2]);
-          __stcs(o + (size_t)(4 * i2) * C, r.a.x);
-          __stcs(o + (size_t)(4 * i2 + 1) * C, r.a.y);
-          __stcs(o + (size_t)(4 * i2 + 2) * C, r.b.x);
-          __stcs(o + (size_t)(4 * i2 + 3) * C, r.b.y);
-        }
-      }
-      return;
-    }
     const F4 Ds = scale4(D, s);
     if constexpr (OUT == kOutBranch) {
       F4 I[4];
@@ -581,91 +541,6 @@ __global__ void __launch_bounds__(256, 1) k_tree4(const KParams P) {
                  : "memory");
 }
 
-// Persistent serving kernel over a flattened (job, column-tile) queue: the
-// columns of many small A = 4 jobs in one launch.  Each CTA owns all 512
-// tensor-memory columns for its lifetime, claims work items one at a time,
-// reloads the tables when the claimed item belongs to another job than the
-// previous one, and runs the same per-warp column code as k_tree4, so every
-// column's result equals that of a separate call.  A claim past the
-// published items waits (bounded) for more until the queue is closed.
-__device__ __forceinline__ int ld_acquire(const int *p) {
-  int v;
-  asm volatile("ld.acquire.sys.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-template <bool F81, int MASK>
-__global__ void __launch_bounds__(256, 1) k_tree4_packed(const T4Queue Q) {
-  extern __shared__ __align__(16) float sm[];
-  __shared__ uint32_t s_taddr;
-  __shared__ int s_item;
-  const int warp = threadIdx.x >> 5;
-  if (warp == 0) {
-    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&s_taddr);
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(512)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = s_taddr;
-  const int nb = blockDim.x;
-  const int lane = threadIdx.x & 31;
-  const uint32_t tb =
-      tmem_base + (((uint32_t)(warp & 3) * 32u) << 16) + (uint32_t)(warp >> 2) * (512u / (uint32_t)(nb >> 7));
-  int loaded = -1;
-  for (;;) {
-    if (threadIdx.x == 0) {
-      const int it = atomicAdd(Q.head, 1);
-      int avail = ld_acquire(Q.published);
-      for (int polls = 0; it >= avail && !ld_acquire(Q.closed) && polls < Q.wait_polls; ++polls) {
-        __nanosleep(256);
-        avail = ld_acquire(Q.published);
-      }
-      if (it < avail) {
-        s_item = it;
-      } else {
-        // closed and drained: done; still open after the bounded wait: the
-        // wait gave up, which the status word records
-        if (!ld_acquire(Q.closed) && Q.err) atomicAdd(Q.err, 1);
-        s_item = -1;
-      }
-    }
-    __syncwarp();  // bar.sync is warp-aligned: warp 0 whole before it
-    __syncthreads();
-    const int it = s_item;
-    if (it < 0) break;
-    const int4 w = Q.items[it];
-    const KParams &P = Q.jobs[w.x];
-    if (w.x != loaded) {
-      // every thread is past the previous item (barrier above)
-      t4_load(P, sm);
-      __syncthreads();
-      t4_piL(P, sm);
-      __syncthreads();
-      loaded = w.x;
-    }
-    for (int c0 = w.y; c0 < w.z; c0 += nb) t4_cols<F81, MASK, kOutSum>(P, sm, tb, c0 + (int)threadIdx.x - lane);
-    __syncthreads();  // s_item and, on a job change, the tables are rewritten next
-  }
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512)
-                 : "memory");
-}
-
-template <bool F, int M>
-int t4packed(const T4Queue &q, int grid, int block, size_t smem, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_tree4_packed<F, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
-  k_tree4_packed<F, M><<<grid, block, smem, s>>>(q);
-  return (int)cudaGetLastError();
-}
-
 template <bool F, int M, int O>
 int t4launch(const KParams &p, int grid, int block, size_t smem, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(k_tree4<F, M, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -694,14 +569,6 @@ int launch_tree4(const KParams &p, bool f81, int mask_mode, int grid, int block,
                                 : t4launch_m<kOutSum>(p, f81, mask_mode, grid, block, smem, s);
 }
 
-int launch_tree4_packed(const T4Queue &q, bool f81, int mask_mode, int grid, int block, size_t smem,
-                        cudaStream_t s) {
-  if (f81) return mask_mode == kMaskAuto ? t4packed<true, kMaskAuto>(q, grid, block, smem, s)
-                                         : t4packed<true, kMaskNone>(q, grid, block, smem, s);
-  return mask_mode == kMaskAuto ? t4packed<false, kMaskAuto>(q, grid, block, smem, s)
-                                : t4packed<false, kMaskNone>(q, grid, block, smem, s);
-}
-
 int preload_tree4() {
   cudaFuncAttributes a;
   const void *fns[] = {(const void *)k_tree4<false, kMaskAuto, kOutSum>, (const void *)k_tree4<false, kMaskGiven, kOutSum>,
@@ -712,10 +579,6 @@ int preload_tree4() {
     if (e != cudaSuccess) return (int)e;
   }
   return 0;
-}
-
-int launch_tree4_post(const KParams &p, int grid, int block, size_t smem, cudaStream_t s) {
-  return t4launch<false, kMaskNone, kOutPost>(p, grid, block, smem, s);
 }
 
 }  // namespace subby

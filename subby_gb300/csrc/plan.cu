@@ -258,10 +258,13 @@ struct subby_plan {
   int4 *d_prog = nullptr, *d_prog_w = nullptr, *d_prog_s = nullptr;
   // A = 4, inside only (k_inside4): one int4 per internal node
   std::vector<int4> prog_i;
+  std::vector<int> prog_other;   // per step: the step of the child that waits on the stack, or -1
   int prog_i_slots = 0;
   int4 *d_prog_i = nullptr;
+  int *d_prog_other = nullptr;
   uint8_t *d_leaf = nullptr;          // (R,) 1 for leaves
-  std::vector<float> hVd, hVu;        // FP32 projection matrices (kernel parameters of k_proj)
+  std::vector<float> hVd, hVu;        // FP32 projection matrices (kernel parameters of k_proj, k_pass4)
+  float hpi[4] = {0.f, 0.f, 0.f, 0.f};  // A = 4: FP32 pi (k_pass4)
   std::vector<double> V, mu, pi, t;   // FP64 model and branch lengths (host)
   float f81_mu = 0.f;
   int f81_model = 0;   // M(t) has the F81 / JC closed form (checked on the host)
@@ -576,7 +579,7 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
       need[v] = (li && ri) ? std::max(a, b + 1) : a;
     }
     P->prog_i_slots = need[0];
-    std::vector<int> slot_of(R, -1);
+    std::vector<int> slot_of(R, -1), step_of(R, -1);
     std::vector<std::pair<int, int>> st;   // node, state (0: enter, 1: first child done, 2: both)
     int sp = 0, last = -1;
     st.push_back({0, 0});
@@ -606,6 +609,8 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
       }
       auto ref = [&](int c) { return left[c] < 0 ? c : c == last ? INT_MIN : ~slot_of[c]; };
       P->prog_i.push_back(make_int4(v, ref(l), ref(r), -1));
+      P->prog_other.push_back(slot_of[first] >= 0 ? step_of[first] : -1);
+      step_of[v] = (int)P->prog_i.size() - 1;
       if (slot_of[first] >= 0) --sp;
       last = v;
       st.pop_back();
@@ -765,6 +770,11 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(P->d_prog_i, P->prog_i.data(), sizeof(int4) * P->prog_i.size(), cudaMemcpyHostToDevice,
                             qs);
+      if (e == cudaSuccess)
+        e = pool_alloc((void **)&P->d_prog_other, sizeof(int) * P->prog_other.size(), P->pool, qs);
+      if (e == cudaSuccess)
+        e = cudaMemcpyAsync(P->d_prog_other, P->prog_other.data(), sizeof(int) * P->prog_other.size(),
+                            cudaMemcpyHostToDevice, qs);
     }
     std::vector<uint8_t> leaf((size_t)R);
     for (int n = 0; n < R; ++n) leaf[n] = left[n] < 0;
@@ -774,6 +784,8 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
   }
   P->hVd.assign(hsm.begin() + (o.Vd - o.Vu), hsm.begin() + (o.Vd - o.Vu) + A * A);
   P->hVu.assign(hsm.begin(), hsm.begin() + A * A);
+  if (A == 4)
+    for (int a = 0; a < 4; ++a) P->hpi[a] = (float)pi[a];
   std::vector<float> hMT, hMN, hGQ;
   std::vector<float2> hcx;
   std::vector<int> grp_br;
@@ -1084,7 +1096,7 @@ int subby_plan_destroy(subby_plan *P) {
   if (s && P->used) cudaStreamWaitEvent(s, P->last_use, 0);
   if (P->s_in) cudaStreamSynchronize(P->s_in);
   if (P->s_out) cudaStreamSynchronize(P->s_out);
-  void *bufs[] = {P->d_tab, P->d_tab64, P->d_steps, P->d_slots, P->d_prog, P->d_prog_w, P->d_prog_s, P->d_prog_i, P->d_leaf, P->d_cxu, P->d_tab16, P->d_err,
+  void *bufs[] = {P->d_tab, P->d_tab64, P->d_steps, P->d_slots, P->d_prog, P->d_prog_w, P->d_prog_s, P->d_prog_i, P->d_prog_other, P->d_leaf, P->d_cxu, P->d_tab16, P->d_err,
                   P->d_cx, P->d_grp_br, P->d_gq};
   for (void *b : bufs)
     if (b) cudaFreeAsync(b, s);
@@ -1426,6 +1438,41 @@ int plan_inside4(subby_plan *P, int mode, int C, Launch &L) {
   return 0;
 }
 
+// A = 4 with an outside pass (k_pass4): summed counts, or posteriors (post).
+// Returns 1 when it does not apply.
+int plan_pass4(subby_plan *P, int mode, bool post, int C, Launch &L) {
+  if (P->A != 4 || g_kernel_sel != 0 || P->R < 2 || (!post && !(mode & kModeCounts)) ||
+      (mode & (kModeGrad | kModeBranch)) || (int)P->prog_i.size() > pass4_steps())
+    return 1;
+  int maxsm = 0;
+  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, P->device);
+  KParams &k = L.kp;
+  k.nsteps = (int)P->prog_i.size();
+  k.nslots = P->prog_i_slots;
+  const bool f81 = (mode & kModeF81) != 0;
+  // two columns per thread once one each would take a second wave (384
+  // threads per SM)
+  L.columns = C > 384 * P->nsm ? 2 : 1;
+  auto bytes = [&](int block) { return pass4_smem(P->R, k.nslots, block, L.columns, f81, post); };
+  // three CTAs of 128 threads per SM when their tables fit, else one CTA of
+  // as many threads (up to 384) as fit beside one copy
+  L.block = 128;
+  int per_sm = 3;
+  if (3 * (bytes(128) + 1024) > (size_t)maxsm + 1024) {
+    per_sm = 1;
+    L.block = 384;
+    while (L.block > 32 && bytes(L.block) > (size_t)maxsm) L.block -= 32;
+    if (bytes(L.block) > (size_t)maxsm) return 1;
+  }
+  while (L.block > 32 && C < P->nsm * L.block * L.columns) L.block = (L.block / 2 + 31) / 32 * 32;
+  L.smem = bytes(L.block);
+  L.kernel = 5;
+  L.small = false;
+  L.grid = std::max(1, std::min((C + L.block * L.columns - 1) / (L.block * L.columns), P->nsm * per_sm));
+  L.nworkers = L.grid * L.block;
+  return 0;
+}
+
 // Large alphabets (A = 16, 20, 32, 64): k_walk (tree walk, 128 columns per
 // CTA, stored-node slots in global memory) then, for Counts, k_acc over the
 // staged per-branch vectors.  Columns are processed in chunks so that the
@@ -1602,33 +1649,46 @@ int run_post(subby_plan *P, const int32_t *d_aln, int C, int node, float *d_node
   if (all && d_br) CU(cudaMemsetAsync(d_br, 0, (size_t)A * A * C * sizeof(float), stream));
   const bool outside = R > 1 && node != 0;
   if (!outside && !d_node) return mark_use(P, stream);
-  Launch L4;
-  if (A == 4 && R > 1 && plan_tree4(P, 0, C, L4) == 0) {
-    // the A = 4 tree-program kernel writes both posteriors directly
-    KParams &k = L4.kp;
-    k.aln = d_aln;
-    k.C = C;
-    k.R = R;
-    k.A = A;
-    k.nInt = P->nInt;
-    k.mode = (node <= 0 && d_node) ? kModeRootProb : 0;
-    k.mask_mode = kMaskNone;
-    k.tab = P->d_tab;
-    k.tab64 = P->d_tab64;
-    k.off = P->off;
-    k.steps = P->d_steps;
-    k.slots = P->d_slots;
-    k.root_is_leaf = P->root_is_leaf;
-    k.f81_mu = P->f81_mu;
-    k.nworkers = L4.nworkers;
-    k.rootp = node <= 0 ? d_node : nullptr;
-    k.npost = d_node;
-    k.npost_node = node;
-    k.bpost = d_br;
-    const int lr = launch_tree4_post(k, L4.grid, L4.block, L4.smem, stream);
-    if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("kernel launch failed: ") + cudaGetErrorString((cudaError_t)lr));
-    g_launches += 1;
-    return mark_use(P, stream);
+  if (A == 4 && R > 1) {
+    // directly from the A = 4 kernels: the root alone without an outside pass
+    Launch L4;
+    const int m4 = (node <= 0 && d_node) ? kModeRootProb : 0;
+    const bool root_only = node == 0 && plan_inside4(P, m4, C, L4) == 0;
+    if (root_only || (node != 0 && plan_pass4(P, 0, true, C, L4 = Launch()) == 0)) {
+      KParams &k = L4.kp;
+      k.aln = d_aln;
+      k.C = C;
+      k.R = R;
+      k.A = A;
+      k.nInt = P->nInt;
+      k.mode = m4;
+      k.mask_mode = kMaskNone;
+      k.tab = P->d_tab;
+      k.tab64 = P->d_tab64;
+      k.off = P->off;
+      k.root_is_leaf = P->root_is_leaf;
+      k.f81_mu = P->f81_mu;
+      k.nworkers = L4.nworkers;
+      k.rootp = node <= 0 ? d_node : nullptr;
+      k.npost = d_node;
+      k.npost_node = node;
+      k.bpost = d_br;
+      int lr;
+      if (root_only) {
+        lr = launch_inside4(k, L4.columns, L4.grid, L4.block, L4.smem, stream);
+      } else {
+        const size_t n4 = (size_t)k.nsteps * L4.columns * L4.nworkers;
+        int rc;
+        if ((rc = P->grow(P->work, al256(n4 * 16) + n4 * 4 + 256, stream))) return rc;
+        k.scrV = (float *)P->work.p;
+        k.scrW = (int *)((char *)P->work.p + al256(n4 * 16));
+        lr = launch_pass4(k, P->prog_i.data(), P->prog_other.data(), P->hVd.data(), P->hVu.data(), P->hpi, false, kMaskNone, true, L4.columns, L4.grid,
+                          L4.block, L4.smem, stream);
+      }
+      if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("kernel launch failed: ") + cudaGetErrorString((cudaError_t)lr));
+      g_launches += 1;
+      return mark_use(P, stream);
+    }
   }
   const bool stage = outside && d_br;
   const int mode = (node <= 0 && d_node) ? kModeRootProb : 0;
@@ -1938,9 +1998,11 @@ int run_common(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float 
   const bool tree = tree_supported(P->A) && !(mode & kModeGrad) && g_kernel_sel != 1;
   const bool small = small_supported(P->A);
   int rc;
-  bool tree4 = false, inside4 = false;
+  bool tree4 = false, inside4 = false, p4 = false;
   if (tree && plan_inside4(P, mode, C, L) == 0) {
     inside4 = true;
+  } else if (tree && plan_pass4(P, mode, false, C, L = Launch()) == 0) {
+    p4 = true;
   } else if (tree && (rc = plan_tree4(P, mode, C, L = Launch())) == 0) {
     tree4 = true;
   } else {
@@ -1973,14 +2035,17 @@ int run_common(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float 
   k.grad_C = d_gC;
   // scratch
   const size_t nsl = (size_t)std::max(tree ? P->prog_slots : P->nslots, 1);
-  const size_t vbytes = (tree && !L.global_slots) ? 0 : nsl * L.nworkers * P->A * sizeof(float);
-  const size_t wbytes = (tree && !L.global_slots) ? 0 : nsl * L.nworkers * 2 * sizeof(int);
+  const size_t p4n = p4 ? (size_t)k.nsteps * L.columns * L.nworkers : 0;
+  const size_t vbytes = p4 ? p4n * 16 : (tree && !L.global_slots) ? 0 : nsl * L.nworkers * P->A * sizeof(float);
+  const size_t wbytes = p4 ? p4n * 4 : (tree && !L.global_slots) ? 0 : nsl * L.nworkers * 2 * sizeof(int);
   const size_t vb_al = (vbytes + 255) & ~(size_t)255;
   if ((rc = P->grow(P->work, vb_al + wbytes + 256, stream))) return rc;
   k.scrV = (float *)P->work.p;
   k.scrW = (int *)((char *)P->work.p + vb_al);
   if (grid_out) *grid_out = L.grid;
-  int lr = inside4 ? launch_inside4(k, L.columns, L.grid, L.block, L.smem, stream)
+  int lr = p4 ? launch_pass4(k, P->prog_i.data(), P->prog_other.data(), P->hVd.data(), P->hVu.data(), P->hpi, (mode & kModeF81) != 0, mask_mode, false,
+                             L.columns, L.grid, L.block, L.smem, stream)
+           : inside4 ? launch_inside4(k, L.columns, L.grid, L.block, L.smem, stream)
            : tree4 ? launch_tree4(k, (mode & kModeF81) != 0, mask_mode, L.grid, L.block, L.smem, stream)
            : tree ? launch_tree(k, P->A, L.store, L.grid, L.block, L.smem, stream)
            : small ? launch_small(k, P->A, L.grid, L.block, L.smem, stream)
@@ -1994,16 +2059,16 @@ int run_common(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float 
 }  // namespace
 
 namespace subby {
-// Packed serving (server.cu): the A = 4 tree kernel's parameters of a
-// device-pointer run of plan P over d_aln (R, C), without launching.  On
-// success `stream` waits for the plan's tables and *smem / *block are the
-// launch's dynamic shared memory and CTA size; the caller launches the
-// packed kernel on `stream` and then calls plan_mark_used.  Returns nonzero
-// (nothing enqueued) when the plan does not take the A = 4 tree kernel with
-// 256 threads per CTA, or the kernel selector is not automatic.
-int plan_tree4_params(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_counts,
-                      float *d_root, int counts_kind, int mask_mode, KParams *out, size_t *smem, int *block,
-                      cudaStream_t stream) {
+// Packed serving (server.cu): the parameters of a device-pointer run of plan
+// P over d_aln (R, C) on the packed A = 4 kernel, without launching.  On
+// success `stream` waits for the plan's tables and *smem is the launch's
+// dynamic shared memory; the caller launches the packed kernel on `stream`
+// and then calls plan_mark_used.  Returns nonzero (nothing enqueued) when a
+// run of the plan does not take k_pass4 (or k_inside4), whose columns the
+// packed kernel computes alike, or the kernel selector is not automatic.
+int plan_packed_params(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_counts,
+                       float *d_root, int counts_kind, int mask_mode, KParams *out, size_t *smem,
+                       cudaStream_t stream) {
   if (!P || P->irrev || P->rows || P->A != 4 || P->R < 2 || C < 1 || !out) return SUBBY_ERR_UNSUPPORTED;
   if (mask_mode != SUBBY_MASK_NONE && mask_mode != SUBBY_MASK_AUTO) return SUBBY_ERR_UNSUPPORTED;
   int mode = kModeBT64;
@@ -2014,8 +2079,14 @@ int plan_tree4_params(subby_plan *P, const int32_t *d_aln, int C, float *d_logL,
   if (!d_counts) mask_mode = SUBBY_MASK_NONE;
   std::lock_guard<std::mutex> g(P->lock);
   Launch L;
-  if (plan_tree4(P, mode, C, L) != 0 || L.block != 256) return SUBBY_ERR_UNSUPPORTED;
+  if (plan_pass4(P, mode | kModeCounts, false, C, L) != 0) return SUBBY_ERR_UNSUPPORTED;
   KParams &k = L.kp;
+  const size_t need = pass4_packed_smem(P->R, k.nsteps, k.nslots, (mode & kModeF81) != 0);
+  int maxsm = 0;
+  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, P->device);
+  if (need + 1024 > (size_t)maxsm) return SUBBY_ERR_UNSUPPORTED;
+  k.prog = P->d_prog_i;
+  k.prog_other = P->d_prog_other;
   k.aln = d_aln;
   k.C = C;
   k.R = P->R;
@@ -2027,18 +2098,14 @@ int plan_tree4_params(subby_plan *P, const int32_t *d_aln, int C, float *d_logL,
   k.tab = P->d_tab;
   k.tab64 = P->d_tab64;
   k.off = P->off;
-  k.steps = P->d_steps;
-  k.slots = P->d_slots;
   k.root_is_leaf = P->root_is_leaf;
   k.f81_mu = P->f81_mu;
-  k.nworkers = L.nworkers;
   k.logL = d_logL;
   k.counts = d_counts;
   k.rootp = d_root;
   if (cudaStreamWaitEvent(stream, P->ready, 0) != cudaSuccess) return SUBBY_ERR_CUDA;
   *out = k;
-  *smem = L.smem;
-  *block = L.block;
+  *smem = need;
   return SUBBY_OK;
 }
 

@@ -12,7 +12,7 @@
 //    resident in an LRU cache keyed by a hash of tree and model;
 //  * short A = 4 jobs waiting together run as one launch of the persistent
 //    packed kernel over their flattened (job, 256-column tile) queue
-//    (k_tree4_packed);
+//    (k_pass4_packed);
 //  * every other job is admitted when one of `max_inflight` slots is free
 //    and its device footprint fits the budget; among waiting jobs the one
 //    with the smallest estimated device time goes first, less a credit that
@@ -55,14 +55,15 @@
 
 namespace subby {
 int plan_status_async(subby_plan *P, int *h, cudaStream_t s);
-int plan_tree4_params(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_counts,
-                      float *d_root, int counts_kind, int mask_mode, KParams *out, size_t *smem, int *block,
-                      cudaStream_t stream);
+int plan_packed_params(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_counts,
+                       float *d_root, int counts_kind, int mask_mode, KParams *out, size_t *smem,
+                       cudaStream_t stream);
 int plan_mark_used(subby_plan *P, cudaStream_t stream);
 }  // namespace subby
 
 using subby::KParams;
-using subby::T4Queue;
+using subby::P4Queue;
+using subby::kPackBlock;
 
 namespace {
 
@@ -248,6 +249,7 @@ size_t job_bytes(int R, int C, int A) {
   const size_t outputs = (size_t)4 * C * (A * A + A + 1);
   const size_t scratch = A >= 16 ? std::min<size_t>((size_t)4 << 30, (size_t)8 * (R - 1) * A * C) +
                                        (size_t)4 * R * (A + 1) * std::min(C, 152 * 128)
+                         : A == 4 ? (size_t)10 * R * std::min(C, 152 * 768)  // a node slot per step and resident column
                                  : (size_t)4 * R * (A + 2) * std::min(C, 152 * 256);
   return tables + tokens + outputs + scratch;
 }
@@ -408,6 +410,8 @@ int launch(subby_server *S, SJob *j) {
   return SUBBY_OK;
 }
 
+constexpr size_t kPackScratch = size_t(256) << 20;   // node slots of one packed launch
+
 int pack_tiles(const subby_server *S, int R) { return S->pack_tiles_r[R <= 64 ? 0 : R <= 256 ? 1 : 2]; }
 
 bool packable(const subby_server *S, const SJob *j) {
@@ -451,13 +455,15 @@ int launch_batch(subby_server *S, std::vector<SJob *> &batch) {
   std::vector<size_t> o_tok(n), o_out(n);
   size_t off = 0;
   long long ntiles = 0;
+  int max_steps = 1;   // internal nodes of the largest tree
   for (int i = 0; i < n; ++i) {
     const subby_job &d = batch[i]->d;
     o_tok[i] = off;
     off += align256((size_t)4 * d.R * d.C);
     o_out[i] = off;
     off += align256((size_t)4 * d.C) + align256((size_t)64 * d.C) + align256((size_t)16 * d.C);
-    ntiles += (d.C + 255) / 256;
+    ntiles += (d.C + kPackBlock - 1) / kPackBlock;
+    max_steps = std::max(max_steps, (d.R - 1) / 2);
   }
   const size_t o_kp = off;
   off += align256(sizeof(KParams) * n);
@@ -465,6 +471,13 @@ int launch_batch(subby_server *S, std::vector<SJob *> &batch) {
   off += align256(sizeof(int4) * ntiles);
   const size_t o_ints = off;
   off += 256;
+  // the CTAs' node slots: two CTAs per SM, fewer for trees whose slots would
+  // take more than kPackScratch
+  const size_t per_cta = (size_t)max_steps * kPackBlock;
+  const long long most = std::max<long long>(1, (long long)(kPackScratch / (per_cta * 20)));
+  const int grid_max = (int)std::min({ntiles, 2LL * S->nsm, most});
+  const size_t o_scr = off;
+  off += align256((size_t)grid_max * per_cta * 16) + align256((size_t)grid_max * per_cta * 4);
   if (grow_arena(S, sl, off, st)) return bail(SUBBY_ERR_NOMEM);
   char *base = static_cast<char *>(sl.arena);
   // host staging: parameters, items, queue words, then the row maps
@@ -499,9 +512,8 @@ int launch_batch(subby_server *S, std::vector<SJob *> &batch) {
                       ? reinterpret_cast<float *>(base + o_out[i] + align256((size_t)4 * d.C) +
                                                   align256((size_t)64 * d.C)) : nullptr;
     size_t sm_i = 0;
-    int block = 0;
-    if (subby::plan_tree4_params(plans[i], d_tok, d.C, d_ll, d_ct, d_rp, d.counts_kind, mask, &hkp[njobs], &sm_i,
-                                 &block, st) != 0) {
+    if (subby::plan_packed_params(plans[i], d_tok, d.C, d_ll, d_ct, d_rp, d.counts_kind, mask, &hkp[njobs], &sm_i,
+                                  st) != 0) {
       j->nopack = true;   // runs on the one-job path instead
       continue;
     }
@@ -514,7 +526,7 @@ int launch_batch(subby_server *S, std::vector<SJob *> &batch) {
     }
     const int rc = subby_gather_rows(d.alignment, d.pitch, rowmap, d.R, d.C, d_tok, st);
     if (rc) return bail(rc);
-    const int span = 256 * pack_tiles(S, d.R);
+    const int span = kPackBlock * pack_tiles(S, d.R);
     for (int c0 = 0; c0 < d.C; c0 += span) hit[nit++] = make_int4(njobs, c0, std::min(d.C, c0 + span), 0);
     const bool want_k[3] = {d_ll != nullptr, d_ct != nullptr, d_rp != nullptr};
     const size_t n_out[3] = {(size_t)4 * d.C, (size_t)64 * d.C, (size_t)16 * d.C};
@@ -532,10 +544,11 @@ int launch_batch(subby_server *S, std::vector<SJob *> &batch) {
   cudaError_t e = cudaMemcpyAsync(base + o_kp, hs, o_ints + 256 - o_kp, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return bail(SUBBY_ERR_CUDA);
   int *d_q = reinterpret_cast<int *>(base + o_ints);
-  const T4Queue q{reinterpret_cast<const KParams *>(base + o_kp), reinterpret_cast<const int4 *>(base + o_items),
-                  d_q, d_q + 1, d_q + 2, 1, d_q + 3};
-  const int grid = (int)std::min<long long>(nit, S->nsm);
-  if (subby::launch_tree4_packed(q, f81, mask, grid, 256, smem, st) != 0) return bail(SUBBY_ERR_CUDA);
+  const P4Queue q{reinterpret_cast<const KParams *>(base + o_kp), reinterpret_cast<const int4 *>(base + o_items),
+                  d_q, d_q + 1, d_q + 2, 1, d_q + 3, max_steps, reinterpret_cast<float4 *>(base + o_scr),
+                  reinterpret_cast<int *>(base + o_scr + align256((size_t)grid_max * per_cta * 16))};
+  const int grid = (int)std::min<long long>(nit, grid_max);
+  if (subby::launch_pass4_packed(q, f81, mask, grid, smem, st) != 0) return bail(SUBBY_ERR_CUDA);
   for (int i = 0; i < njobs; ++i) {
     SJob *j = taken[i];
     const KParams &k = hkp[i];
@@ -853,19 +866,17 @@ int subby_server_stats(subby_server *S, double *engine_busy_s, int *plans_cached
 
 int subby_debug_packed_queue_wait(int polls, int grid, int *gave_up) {
   if (polls < 1 || polls > 100000 || grid < 1 || !gave_up) return SUBBY_ERR_ARG;
-  int dev = 0, nsm = 0, maxsm = 0;
+  int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   grid = std::min(grid, nsm);
   int *d = nullptr;
   if (cudaMalloc(&d, 4 * sizeof(int)) != cudaSuccess) return SUBBY_ERR_NOMEM;
   // an open queue with nothing published: every CTA's claim waits and gives up
   cudaError_t e = cudaMemset(d, 0, 4 * sizeof(int));
-  const T4Queue q{nullptr, nullptr, d, d + 1, d + 2, polls, d + 3};
+  const P4Queue q{nullptr, nullptr, d, d + 1, d + 2, polls, d + 3, 1, nullptr, nullptr};
   if (e == cudaSuccess) {
-    // at least half the SM's shared memory: one CTA (owner of the tensor memory) per SM
-    const int lr = subby::launch_tree4_packed(q, false, SUBBY_MASK_AUTO, grid, 256, (size_t)(maxsm / 2 + 4096), 0);
+    const int lr = subby::launch_pass4_packed(q, false, SUBBY_MASK_AUTO, grid, 1024, 0);
     e = lr ? (cudaError_t)lr : cudaDeviceSynchronize();
   }
   int h[4] = {0, 0, 0, 0};

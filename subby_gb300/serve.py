@@ -140,6 +140,8 @@ def job_device_bytes(R: int, C: int, A: int) -> int:
     outputs = 4 * C * (A * A + A + 1)
     if A >= 16:
         scratch = min(STAGE_CAP, 8 * (R - 1) * A * C) + 4 * R * (A + 1) * min(C, 152 * 128)
+    elif A == 4:   # a node slot per step and resident column
+        scratch = 10 * R * min(C, 152 * 768)
     else:
         scratch = 4 * R * (A + 2) * min(C, 152 * 256)
     return tables + tokens + outputs + scratch
