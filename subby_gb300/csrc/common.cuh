@@ -136,7 +136,6 @@ bool tree_supported(int A);
 // A = 64 walk, large-alphabet accumulation (k_big.cu)
 bool big_supported(int A);
 int big_tile();
-int big_acc_group(int A);
 // mode: 0 inside pass only (LogLike / RootProb), 1 stage eigen vectors, 2 stage F81 vectors
 int launch_walk(const KParams &p, int A, int mode, bool tc, float *sa, float *sb, int c_base, int c_count,
                 int grid, cudaStream_t s);
@@ -181,7 +180,7 @@ int launch_post(const KParams &p, int A, const float *sa, const float *sb, int c
                 int n_hi, int row_off, float *br_out, int grid, cudaStream_t s);
 // tc: A = 64 eigen back-transform on the tensor cores
 int launch_acc(const KParams &p, int A, bool f81, bool tc, const float *sa, const float *sb, int c_base,
-               int c_count, int grid, cudaStream_t s);
+               int c_count, int nsm, cudaStream_t s);
 int launch_tree4(const KParams &p, bool f81, int mask_mode, int grid, int block, size_t smem,
                  cudaStream_t s);
 // A = 4 inside pass only (k_inside4.cu): LogLike / RootProb

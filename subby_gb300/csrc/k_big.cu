@@ -23,6 +23,8 @@
 // V C V^T (oracle.py:1087-1137) through shared memory and writes counts.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "walk.cuh"
 
@@ -31,23 +33,24 @@ namespace {
 
 // ---------------------------------------------------------------------------
 // Kernel 2: accumulation over branches + back-transform, G columns per CTA.
-// Thread t: 4 x 4 block b = t % NB of (k, l), column group t / NB of 8 columns.
-template <int A>
+// Thread t: 4 x 4 block b = t % NB of (k, l), column group t / NB of Q columns.
+template <int A, int Q = 8>
 struct AccGeo {
   static constexpr int KB = A / 4;          // blocks per side
   static constexpr int NB = KB * KB;        // (k, l) blocks
-  static constexpr int GROUPS = 256 / NB;   // column groups of 8
-  static constexpr int G = GROUPS * 8;      // columns per CTA
+  static constexpr int GROUPS = 256 / NB;   // column groups
+  static constexpr int G = GROUPS * Q;      // columns per CTA
   static constexpr int THREADS = NB * GROUPS;
 };
 
 // Stages of the k_acc ring: as many (J_n, a, b) buffers as fit in the
 // G x A x A floats of the back-transform buffer, at most 8.
-template <int A>
+template <int A, int Q = 8>
 struct AccRing {
-  static constexpr int STAGE = A * A + 2 * AccGeo<A>::G * A;       // floats per stage
-  static constexpr int CBUF = AccGeo<A>::G * A * A;                // back-transform buffer
-  static constexpr int S = (CBUF / STAGE) < 8 ? (CBUF / STAGE) : 8;
+  static constexpr int STAGE = A * A + 2 * AccGeo<A, Q>::G * A;    // floats per stage
+  static constexpr int CBUF = AccGeo<A, Q>::G * A * A;             // back-transform buffer
+  static constexpr int FIT = CBUF / STAGE;
+  static constexpr int S = FIT < 4 ? 4 : FIT < 8 ? FIT : 8;
   static constexpr int SCAL = (S * STAGE > CBUF ? S * STAGE : CBUF);  // F81 scalars after both
   static_assert(S >= 3, "ring too short");
 };
@@ -64,11 +67,13 @@ __host__ __device__ constexpr int acc_vv_offset() {
 // tensor-core Counts); otherwise on CUDA cores.
 // PB: per-branch counts — each work item is one (branch, column group) and
 // writes that branch's counts (R, A, A, C layout) instead of summing.
-template <int A, bool F81, bool TCB, bool PB = false>
+// Q: columns per thread (8; 2 for few columns, see acc_columns).
+template <int A, bool F81, bool TCB, bool PB = false, int Q = 8>
 __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__restrict__ stage_a,
                                                  const float *__restrict__ stage_b, int c_base, int c_count) {
-  using Gm = AccGeo<A>;
-  using Rg = AccRing<A>;
+  using Gm = AccGeo<A, Q>;
+  using Rg = AccRing<A, Q>;
+  static_assert(Q == 8 || (!F81 && !TCB && !PB), "short column groups: summed eigen counts");
   static_assert(!(PB && TCB), "per-branch counts use the CUDA-core back-transform");
   static_assert(!TCB || (A == 64 && !F81), "tensor-core back-transform is A = 64 eigen");
   constexpr int G = Gm::G;
@@ -102,14 +107,14 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
   // output row r, the 8 columns col0.. of this thread's group: two 16-byte
   // stores when the rows are 16-byte aligned and all 8 columns exist
   const bool vec_out = (C & 3) == 0 && (c_base & 3) == 0;
-  auto store8 = [&](size_t r, const float (&v)[8], int col0, int ncols) {
+  auto storeq = [&](size_t r, const float (&v)[Q], int col0, int ncols) {
     float *o = cbase + r * C + col0;
-    if (vec_out && ncols >= 8) {
-      *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
-      *reinterpret_cast<float4 *>(o + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    if (Q == 8 && vec_out && ncols >= 8) {
+      *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1 % Q], v[2 % Q], v[3 % Q]);
+      *reinterpret_cast<float4 *>(o + 4) = make_float4(v[4 % Q], v[5 % Q], v[6 % Q], v[7 % Q]);
     } else {
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
+      for (int q = 0; q < Q; ++q)
         if (q < ncols) o[q] = v[q];
     }
   };
@@ -169,7 +174,7 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
     const int g0 = gi * G;                       // first column (chunk-relative)
     const int gcols = min(G, c_count - g0);
     // accumulators: ac2[a][p][q] = (C[k0+a][l0+2p], C[k0+a][l0+2p+1]) of column q
-    float2 ac2[4][2][8];
+    float2 ac2[4][2][Q];
 #define ACC(a, b, q) (((b) & 1) ? ac2[a][(b) >> 1][q].y : ac2[a][(b) >> 1][q].x)
     // F81: per-column h (rows), g (columns) and z, one element set per thread
     constexpr int NE = (G * A + 255) / 256;
@@ -179,7 +184,7 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
 #pragma unroll
       for (int pp = 0; pp < 2; ++pp)
 #pragma unroll
-        for (int q = 0; q < 8; ++q) ac2[a][pp][q] = make_float2(0.f, 0.f);
+        for (int q = 0; q < Q; ++q) ac2[a][pp][q] = make_float2(0.f, 0.f);
     if (F81) {
 #pragma unroll
       for (int r = 0; r < NE; ++r) hreg[r] = greg[r] = 0.f;
@@ -276,11 +281,11 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
             jp[a][1] = make_float2(r.z, r.w);
           }
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int cc = grp * 8 + q;
-            // (rot(cc) = rot(q): the groups of 8 columns start at rotation 0)
-            const float4 d = *reinterpret_cast<const float4 *>(da + cc * A + stage_chunk<A>(k0 / 4, stage_rot(A, q)));
-            const float4 u = *reinterpret_cast<const float4 *>(db + cc * A + stage_chunk<A>(l0 / 4, stage_rot(A, q)));
+          for (int q = 0; q < Q; ++q) {
+            const int cc = grp * Q + q;
+            const int rot = stage_rot(A, Q == 8 ? q : cc);   // (groups of 8 start at rotation 0)
+            const float4 d = *reinterpret_cast<const float4 *>(da + cc * A + stage_chunk<A>(k0 / 4, rot));
+            const float4 u = *reinterpret_cast<const float4 *>(db + cc * A + stage_chunk<A>(l0 / 4, rot));
             const float dk[4] = {d.x, d.y, d.z, d.w};
             const float2 up[2] = {make_float2(u.x, u.y), make_float2(u.z, u.w)};
 #pragma unroll
@@ -294,8 +299,8 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
         } else {
           const float4 abg = __ldg(reinterpret_cast<const float4 *>(F8) + n + 1);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int cc = grp * 8 + q;
+          for (int q = 0; q < Q; ++q) {
+            const int cc = grp * Q + q;
             const float4 d = *reinterpret_cast<const float4 *>(da + cc * A + k0);
             const float4 u = *reinterpret_cast<const float4 *>(db + cc * A + l0);
             const float dk[4] = {d.x, d.y, d.z, d.w};
@@ -313,7 +318,7 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
     }
     __syncthreads();
     // ------------------------------------------------------------- epilogue
-    const int col0 = c_base + g0 + grp * 8, ncols = gcols - grp * 8;
+    const int col0 = c_base + g0 + grp * Q, ncols = gcols - grp * Q;
     if (F81) {
       // h, g, z of every column through shared memory to the (k, l) blocks
       float *Hs = pis + A, *Gs = Hs + G * A, *Zs = Gs + G * A;
@@ -335,13 +340,13 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
           for (int b = 0; b < 4; ++b) {
             const int i = k0 + a, j = l0 + b;
             const float pi_i = pis[i], f = (i == j) ? 1.f : mu * pis[j];
-            float v[8];
+            float v[Q];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const int cc = grp * 8 + q;
+            for (int q = 0; q < Q; ++q) {
+              const int cc = grp * Q + q;
               v[q] = f * (ACC(a, b, q) + Hs[cc * A + i] + pi_i * (Gs[cc * A + j] + Zs[cc]));
             }
-            store8((size_t)(i * A + j), v, col0, ncols);
+            storeq((size_t)(i * A + j), v, col0, ncols);
           }
       }
       __syncthreads();
@@ -514,8 +519,8 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
     const float *V = Vs;
     if (active) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int cc = grp * 8 + q;
+      for (int q = 0; q < Q; ++q) {
+        const int cc = grp * Q + q;
 #pragma unroll
         for (int a = 0; a < 4; ++a)
           *reinterpret_cast<float4 *>(Cs + ((size_t)cc * A + k0 + a) * A + l0) =
@@ -530,7 +535,7 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
 #pragma unroll
         for (int pp = 0; pp < 2; ++pp)
 #pragma unroll
-          for (int q = 0; q < 8; ++q) ac2[a][pp][q] = make_float2(0.f, 0.f);
+          for (int q = 0; q < Q; ++q) ac2[a][pp][q] = make_float2(0.f, 0.f);
       for (int l = 0; l < A; l += 4) {
         float2 vjp[2][4];  // (V[j][l+m], V[j+1][l+m]) for the two j pairs of this block
 #pragma unroll
@@ -543,8 +548,8 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
           vjp[pp][3] = make_float2(r0.w, r1.w);
         }
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int cc = grp * 8 + q;
+        for (int q = 0; q < Q; ++q) {
+          const int cc = grp * Q + q;
 #pragma unroll
           for (int a = 0; a < 4; ++a) {
             const float4 cr = *reinterpret_cast<const float4 *>(Cs + ((size_t)cc * A + k0 + a) * A + l);
@@ -562,8 +567,8 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
     __syncthreads();
     if (active) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int cc = grp * 8 + q;
+      for (int q = 0; q < Q; ++q) {
+        const int cc = grp * Q + q;
 #pragma unroll
         for (int a = 0; a < 4; ++a)
           *reinterpret_cast<float4 *>(Cs + ((size_t)cc * A + k0 + a) * A + l0) =
@@ -578,7 +583,7 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
 #pragma unroll
         for (int pp = 0; pp < 2; ++pp)
 #pragma unroll
-          for (int q = 0; q < 8; ++q) ac2[a][pp][q] = make_float2(0.f, 0.f);
+          for (int q = 0; q < Q; ++q) ac2[a][pp][q] = make_float2(0.f, 0.f);
       for (int k = 0; k < A; ++k) {
         float2 vi2[4];
 #pragma unroll
@@ -587,8 +592,8 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
           vi2[a] = make_float2(v, v);
         }
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int cc = grp * 8 + q;
+        for (int q = 0; q < Q; ++q) {
+          const int cc = grp * Q + q;
           const float4 tr = *reinterpret_cast<const float4 *>(Cs + ((size_t)cc * A + k) * A + l0);
           const float2 tp[2] = {make_float2(tr.x, tr.y), make_float2(tr.z, tr.w)};
 #pragma unroll
@@ -604,10 +609,10 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
           for (int b = 0; b < 4; ++b) {
             const int i = k0 + a, j = l0 + b;
             const float f = (i == j) ? 1.f : Ss[i * A + j];
-            float v[8];
+            float v[Q];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[q] = f * ACC(a, b, q);
-            store8((size_t)(i * A + j), v, col0, ncols);
+            for (int q = 0; q < Q; ++q) v[q] = f * ACC(a, b, q);
+            storeq((size_t)(i * A + j), v, col0, ncols);
           }
       }
     }
@@ -632,23 +637,41 @@ int walk_launch(const KParams &p, int mode, float *sa, float *sb, int c_base, in
   return walk_launch1<64, 2, TC, false>(p, sa, sb, c_base, c_count, grid, s);
 }
 
-template <int A, bool F81, bool TCB, bool PB = false>
+template <int A, bool F81, bool TCB, bool PB = false, int Q = 8>
 int acc_launch1(const KParams &p, const float *sa, const float *sb, int c_base, int c_count, int grid,
                 cudaStream_t s) {
-  using Gm = AccGeo<A>;
+  using Gm = AccGeo<A, Q>;
   const size_t smem = TCB ? (size_t)acc_vv_offset<A>() * sizeof(float) + 49152
-                          : (size_t)(AccRing<A>::SCAL + 2 * Gm::G + 2 * A * A + A + 2 * Gm::G * A + Gm::G) *
+                          : (size_t)(AccRing<A, Q>::SCAL + 2 * Gm::G + 2 * A * A + A + 2 * Gm::G * A + Gm::G) *
                                 sizeof(float);
   cudaError_t e =
-      cudaFuncSetAttribute(k_acc<A, F81, TCB, PB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_acc<A, F81, TCB, PB, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  k_acc<A, F81, TCB, PB><<<grid, 256, smem, s>>>(p, sa, sb, c_base, c_count);
+  k_acc<A, F81, TCB, PB, Q><<<grid, 256, smem, s>>>(p, sa, sb, c_base, c_count);
   return (int)cudaGetLastError();
+}
+
+// Columns per thread of the summed eigen counts: two while those groups fit
+// in one wave, so that a call of few columns spreads over the SMs (whole
+// Counts calls, 50 leaves: A = 16, 4003 columns 185 -> 142 us; A = 20, 1000
+// columns 186 -> 155 us); beyond a wave eight, which load J_n once for four
+// times the columns (A = 16, 9728 columns 216 against 224 us).
+template <int A>
+int acc_columns(const KParams &p, bool f81, int c_count, int nsm) {
+  if (A == 64 || f81 || (p.mode & kModeBranch)) return 8;
+  return (c_count + AccGeo<A, 2>::G - 1) / AccGeo<A, 2>::G <= nsm ? 2 : 8;
 }
 
 template <int A>
 int acc_launch(const KParams &p, bool f81, bool tc, const float *sa, const float *sb, int c_base, int c_count,
-               int grid, cudaStream_t s) {
+               int nsm, cudaStream_t s) {
+  const int q = acc_columns<A>(p, f81, c_count, nsm);
+  const int G = AccGeo<A>::G / 8 * q;
+  const long long items = (long long)(c_count + G - 1) / G * ((p.mode & kModeBranch) ? p.R - 1 : 1);
+  const int grid = (int)std::max<long long>(1, std::min<long long>(items, nsm));
+  if constexpr (A != 64) {
+    if (q == 2) return acc_launch1<A, false, false, false, 2>(p, sa, sb, c_base, c_count, grid, s);
+  }
   if (p.mode & kModeBranch)
     return f81 ? acc_launch1<A, true, false, true>(p, sa, sb, c_base, c_count, grid, s)
                : acc_launch1<A, false, false, true>(p, sa, sb, c_base, c_count, grid, s);
@@ -663,16 +686,6 @@ int acc_launch(const KParams &p, bool f81, bool tc, const float *sa, const float
 
 bool big_supported(int A) { return A == 16 || A == 20 || A == 32 || A == 64; }
 int big_tile() { return kTile; }
-int big_acc_group(int A) {
-  switch (A) {
-    case 16: return AccGeo<16>::G;
-    case 20: return AccGeo<20>::G;
-    case 32: return AccGeo<32>::G;
-    case 64: return AccGeo<64>::G;
-    default: return 0;
-  }
-}
-
 int launch_walk(const KParams &p, int A, int mode, bool tc, float *sa, float *sb, int c_base, int c_count,
                 int grid, cudaStream_t s) {
   if (A != 64) return -1;
@@ -681,12 +694,12 @@ int launch_walk(const KParams &p, int A, int mode, bool tc, float *sa, float *sb
 }
 
 int launch_acc(const KParams &p, int A, bool f81, bool tc, const float *sa, const float *sb, int c_base,
-               int c_count, int grid, cudaStream_t s) {
+               int c_count, int nsm, cudaStream_t s) {
   switch (A) {
-    case 16: return acc_launch<16>(p, f81, false, sa, sb, c_base, c_count, grid, s);
-    case 20: return acc_launch<20>(p, f81, false, sa, sb, c_base, c_count, grid, s);
-    case 32: return acc_launch<32>(p, f81, false, sa, sb, c_base, c_count, grid, s);
-    case 64: return acc_launch<64>(p, f81, tc, sa, sb, c_base, c_count, grid, s);
+    case 16: return acc_launch<16>(p, f81, false, sa, sb, c_base, c_count, nsm, s);
+    case 20: return acc_launch<20>(p, f81, false, sa, sb, c_base, c_count, nsm, s);
+    case 32: return acc_launch<32>(p, f81, false, sa, sb, c_base, c_count, nsm, s);
+    case 64: return acc_launch<64>(p, f81, tc, sa, sb, c_base, c_count, nsm, s);
     default: return -1;
   }
 }

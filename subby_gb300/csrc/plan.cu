@@ -1624,11 +1624,8 @@ int run_big(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_
         if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("projection launch failed: ") + cudaGetErrorString((cudaError_t)lr));
         g_launches += 1;
       }
-      const int G = big_acc_group(A);
-      const long long items = (long long)(cc + G - 1) / G * ((mode & kModeBranch) ? (R - 1) : 1);
-      const int agrid = (int)std::max<long long>(1, std::min<long long>(items, P->nsm));
-      lr = f81tc ? launch_acc_f81_tc(k, sa, sb, k.stage_c, c0, cc, agrid, stream)
-                 : launch_acc(k, A, (mode & kModeF81) != 0, tcb, sa, sb, c0, cc, agrid, stream);
+      lr = f81tc ? launch_acc_f81_tc(k, sa, sb, k.stage_c, c0, cc, std::min((cc + 7) / 8, P->nsm), stream)
+                 : launch_acc(k, A, (mode & kModeF81) != 0, tcb, sa, sb, c0, cc, P->nsm, stream);
       if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("accumulate launch failed: ") + cudaGetErrorString((cudaError_t)lr));
       g_launches += 1;
     }
