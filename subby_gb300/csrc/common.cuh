@@ -267,9 +267,9 @@ int launch_xform(const double *X, const double *tab64, int R, int A, double *gra
 // distance gradient from the raw staging: grad_t[n] += sum_c g_c (D s)^T G_n U
 int launch_grad_cx(const KParams &p, int A, const float *sa, const float *sb, const float *gq, const float *g,
                    int c_base, int c_count, double *grad_t, int grid, cudaStream_t s);
-// A = 64 F81 accumulation on the tensor cores (k_acctc.cu); groups of 8 columns
-int launch_acc_f81_tc(const KParams &p, const float *sa, const float *sb, const float2 *sc, int c_base,
-                      int c_count, int grid, cudaStream_t s);
+// A = 64 F81 accumulation (k_acctc.cu); groups of 8 columns
+int launch_acc_f81_64(const KParams &p, const float *sa, const float *sb, const float2 *sc, int c_base, int c_count,
+                      int grid, cudaStream_t s);
 bool small_supported(int A);
 bool warp_supported(int A);
 int small_block();

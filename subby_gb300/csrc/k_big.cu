@@ -675,7 +675,9 @@ int acc_launch(const KParams &p, bool f81, bool tc, const float *sa, const float
   if (p.mode & kModeBranch)
     return f81 ? acc_launch1<A, true, false, true>(p, sa, sb, c_base, c_count, grid, s)
                : acc_launch1<A, false, false, true>(p, sa, sb, c_base, c_count, grid, s);
-  if (f81) return acc_launch1<A, true, false>(p, sa, sb, c_base, c_count, grid, s);
+  if constexpr (A != 64) {   // (k_acc_f81)
+    if (f81) return acc_launch1<A, true, false>(p, sa, sb, c_base, c_count, grid, s);
+  }
   if constexpr (A == 64) {
     if (tc) return acc_launch1<A, false, true>(p, sa, sb, c_base, c_count, grid, s);
   }

@@ -1598,14 +1598,14 @@ int run_big(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_
   int rc;
   if ((rc = plan_walk(P, k, quad, counts, chunk, H == 2 ? 1 : 2, &w))) return rc;
   const size_t stage_bytes = counts ? al256((size_t)(R - 1) * chunk * A * sizeof(float)) : 0;
-  // A = 64 F81 counts on the tensor cores: per-branch scalars staged too
-  const bool f81tc = counts && (mode & kModeF81) && tc && !(mode & kModeBranch);
-  const size_t stage_c_bytes = f81tc ? al256((size_t)(R - 1) * chunk * sizeof(float2)) : 0;
+  // A = 64 F81 counts (k_acc_f81): per-branch scalars staged too
+  const bool f81_64 = A == 64 && counts && (mode & kModeF81) && !(mode & kModeBranch);
+  const size_t stage_c_bytes = f81_64 ? al256((size_t)(R - 1) * chunk * sizeof(float2)) : 0;
   if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * stage_bytes + stage_c_bytes + 256, stream))) return rc;
   char *base = place_walk(k, w, P->work.p);
   float *sa = (float *)base;
   float *sb = (float *)(base + stage_bytes);
-  k.stage_c = f81tc ? (float2 *)(base + 2 * stage_bytes) : nullptr;
+  k.stage_c = f81_64 ? (float2 *)(base + 2 * stage_bytes) : nullptr;
   const int wmode = counts ? ((mode & kModeF81) ? 2 : 1) : 0;
   if (!counts && (mode & kModeCounts)) {
     // a single-node tree has no branch: counts are zero
@@ -1614,7 +1614,7 @@ int run_big(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_
   }
   for (int c0 = 0; c0 < C; c0 += chunk) {
     const int cc = std::min(chunk, C - c0);
-    int lr = w.q ? launch_qwalk(k, A, w.f81, counts, sa, sb, eigen ? kQRotate : kQLeafU, c0, cc, w.g, stream)
+    int lr = w.q ? launch_qwalk(k, A, w.f81, counts, sa, sb, eigen ? kQRotate : f81_64 ? 0 : kQLeafU, c0, cc, w.g, stream)
                  : launch_walk(k, A, wmode, tc, sa, sb, c0, cc, w.grid, stream);
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("walk launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
@@ -1624,7 +1624,7 @@ int run_big(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_
         if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("projection launch failed: ") + cudaGetErrorString((cudaError_t)lr));
         g_launches += 1;
       }
-      lr = f81tc ? launch_acc_f81_tc(k, sa, sb, k.stage_c, c0, cc, std::min((cc + 7) / 8, P->nsm), stream)
+      lr = f81_64 ? launch_acc_f81_64(k, sa, sb, k.stage_c, c0, cc, std::min((cc + 7) / 8, P->nsm), stream)
                  : launch_acc(k, A, (mode & kModeF81) != 0, tcb, sa, sb, c0, cc, P->nsm, stream);
       if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("accumulate launch failed: ") + cudaGetErrorString((cudaError_t)lr));
       g_launches += 1;
