@@ -15,8 +15,8 @@
 // keeps column c's h, g, z (lane: two states) from the scalars (pi . U, sum
 // s D) that the walk staged.
 //
-// Bound by latency at 16 warps per SM (issue 44 %, load pipe 47 % active): four
-// branches per barrier.  R = 127, 20011 columns (GB300): 925 us; one branch
+// Bound by latency at 16 warps per SM (issue 48 %, load pipe 51 % active): four
+// branches per barrier.  R = 127, 20011 columns (GB300): 846 us; one branch
 // per barrier 1133 us, 256 threads of two columns so 1045 us.  Products on the
 // tensor cores (split-BF16 operands of two columns, 16 branches per K step)
 // took 1245 us, most of it splitting and storing every branch's operands,

@@ -22,10 +22,11 @@
 // into the eigenbasis, two thirds of the products of a Counts walk, do not
 // depend on the tree order and are left to k_proj.
 // Measured (GB300; walk with the raw staging, against k_walk's eigen
-// staging): A = 20, R = 199, C = 20011 1515 -> 432 us; A = 20, R = 399,
-// C = 50000 5490 -> 1823 us; A = 16, R = 99, C = 4003 368 -> 76 us; A = 32,
+// staging): A = 20, R = 199, C = 20011 1515 -> 414 us; A = 20, R = 399,
+// C = 50000 5490 -> 1683 us; A = 16, R = 99, C = 4003 368 -> 72 us; A = 32,
 // R = 127, C = 16000 1724 -> 430 us; F81 at A = 64, R = 127, C = 20011 1617
-// -> 548 us.  What is left is latency at 8 to 12 warps per SM (issue 40 %
+// -> 484 us.  The product's loop is unrolled whole: by fours it measured 432,
+// 1740 and 82 us (no spills either way).  What is left is latency at 8 to 12 warps per SM (issue 40 %
 // active, load pipe 48 %).  Four columns per lane (255 registers, 8 warps
 // per SM) measured 2074 us at R = 399, C = 50000, 128 registers with two
 // columns per lane 2229 us (spills).
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__((q_threads<CPL, F81M>()), MINB)
       __syncwarp();
 #pragma unroll
       for (int q = 0; q < CPL; ++q) y.fill(q, 0.f);
-#pragma unroll 4
+#pragma unroll
       for (int j = 0; j < A; ++j) {
         V m;   // column 0 only
         m.row(0, T + j * A, sg);
