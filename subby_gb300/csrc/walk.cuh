@@ -96,11 +96,17 @@ struct TcState {
   int *err;         // shared: set when a bounded wait gives up
 };
 
+// A = 64: a warp's 32 columns x 32 states as rows of 128 bytes, row l's
+// 16-byte chunk k at position k ^ (l & 7): a lane's own row and four whole
+// rows per instruction both reach all banks.
+constexpr int kRowBuf = 32 * 32 * 4;   // bytes per warp
+
 template <int A>
 struct Walk {
   static constexpr int H = Geo<A>::H;
   static constexpr int S = Geo<A>::S;
-  int c, h, warp;
+  int c, h, warp, lane;
+  float4 *rows;   // H = 2: this warp's row buffer
   float *xch;     // shared exchange buffer: [2][32 states][128 cols] floats
   int *xmax;      // shared [2][128] ints (exponent-field exchange)
   TcState tcs;    // tensor-core state (per thread copy; used when use_tc)
@@ -238,9 +244,9 @@ struct Walk {
   // Outside-pass products of one branch in a single round trip:
   //   O = MN_n-product of D and dt = Vd-product of D (stacked, N = 128) when
   //   MNg is given, dt alone (N = 64) otherwise; ut = Vu-product of U when U
-  //   is given.  dt is scaled by s and stored to pa, ut to pb (when store).
+  //   is given.  dt is scaled by s and stored to pa, ut to pb (st_rows).
   __device__ __forceinline__ void outside_tc(BV<A> &O, const BV<A> &D, const BV<A> *U, const uint16_t *MNg,
-                                             float s, float *pa, float *pb, bool store) {
+                                             float s, float *pa, float *pb, int nrows) {
     TcState &T = tcs;
     const bool wantO = MNg != nullptr, wantU = U != nullptr;
     if (wantO) load_node_B(MNg);
@@ -266,12 +272,12 @@ struct Walk {
       tm_ld32(t, 64u + 32u * h);
 #pragma unroll
       for (int i = 0; i < 32; ++i) t.v[i] *= s;
-      if (store) st(pa, t);
+      st_rows(pa, nrows, t);
     }
     if (wantU) {
       BV<A> t;
       tm_ld32(t, 128u + 32u * h);
-      if (store) st(pb, t);
+      st_rows(pb, nrows, t);
     }
     if (wantO) tm_ld32(O, 32u * h);
   }
@@ -287,6 +293,75 @@ struct Walk {
 #pragma unroll
     for (int q = 0; q < S / 4; ++q)
       *reinterpret_cast<float4 *>(p + 4 * q) = make_float4(x.v[4 * q], x.v[4 * q + 1], x.v[4 * q + 2], x.v[4 * q + 3]);
+  }
+  // The warp's columns as rows of A floats (p: row 0, this half's states),
+  // nrows of them exist.  Written four rows of 128 bytes per instruction: a
+  // lane that stores its own row touches 32 lines with every 16 bytes.
+  __device__ __forceinline__ void st_rows(float *p, int nrows, const BV<A> &x) const {
+    if constexpr (H == 2) {
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        rows[lane * 8 + (q ^ (lane & 7))] = make_float4(x.v[4 * q], x.v[4 * q + 1], x.v[4 * q + 2], x.v[4 * q + 3]);
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int r = 4 * k + (lane >> 3), ch = lane & 7;
+        const float4 t = rows[r * 8 + (ch ^ (r & 7))];
+        if (r < nrows) *reinterpret_cast<float4 *>(p + (size_t)r * A + 4 * ch) = t;
+      }
+    } else if (lane < nrows) {
+      st(p + (size_t)lane * A, x);
+    }
+  }
+  // row `code` of table T (this half's states) of every column of the warp
+  __device__ __forceinline__ void ld_code(BV<A> &o, const float *T, int code) const {
+    if constexpr (H == 2) {
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int r = 4 * k + (lane >> 3), ch = lane & 7;
+        const int cd = __shfl_sync(0xffffffffu, code, r);
+        rows[r * 8 + (ch ^ (r & 7))] = __ldg(reinterpret_cast<const float4 *>(T + (size_t)cd * A) + ch);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float4 t = rows[lane * 8 + (q ^ (lane & 7))];
+        o.v[4 * q] = t.x, o.v[4 * q + 1] = t.y, o.v[4 * q + 2] = t.z, o.v[4 * q + 3] = t.w;
+      }
+    } else {
+      ld(o, T + (size_t)code * A);
+    }
+  }
+  // ... straight into the columns' rows at p
+  __device__ __forceinline__ void st_code(float *p, int nrows, const float *T, int code) const {
+    if constexpr (H == 2) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int r = 4 * k + (lane >> 3), ch = lane & 7;
+        const int cd = __shfl_sync(0xffffffffu, code, r);
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(T + (size_t)cd * A) + ch);
+        if (r < nrows) *reinterpret_cast<float4 *>(p + (size_t)r * A + 4 * ch) = t;
+      }
+    } else {
+      BV<A> x;
+      ld(x, T + (size_t)code * A);
+      st_rows(p, nrows, x);
+    }
+  }
+  // a slot vector: lane-interleaved 16-byte chunks
+  __device__ __forceinline__ void ld_slot(BV<A> &o, const float4 *p) const {
+#pragma unroll
+    for (int q = 0; q < S / 4; ++q) {
+      const float4 t = p[32 * q];
+      o.v[4 * q] = t.x, o.v[4 * q + 1] = t.y, o.v[4 * q + 2] = t.z, o.v[4 * q + 3] = t.w;
+    }
+  }
+  __device__ __forceinline__ void st_slot(float4 *p, const BV<A> &x) const {
+#pragma unroll
+    for (int q = 0; q < S / 4; ++q)
+      p[32 * q] = make_float4(x.v[4 * q], x.v[4 * q + 1], x.v[4 * q + 2], x.v[4 * q + 3]);
   }
   __device__ __forceinline__ void obs(BV<A> &x, int code) const {
     if (code < A) {
@@ -486,6 +561,8 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
   }
   wk.warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  wk.lane = lane;
+  wk.rows = reinterpret_cast<float4 *>(s_dyn + (TC ? kTcDyn : 0) + wk.warp * kRowBuf);
   wk.c = lane + 32 * (wk.warp & 3);
   wk.h = wk.warp >> 2;
   wk.xch = s_xch;
@@ -502,7 +579,9 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
   const int4 *prog = P.prog;
   const int C = P.C;
   const size_t tile_slots = (size_t)P.nslots * kTile;
-  float *svec = P.scrV + (size_t)blockIdx.x * tile_slots * A;  // [slot][c][A]
+  // slot vectors [slot][warp][16-byte chunk][lane]
+  float4 *svec = reinterpret_cast<float4 *>(P.scrV) + (size_t)blockIdx.x * tile_slots * (A / 4) +
+                 (size_t)wk.warp * (S / 4 * 32) + lane;
   // slot words (exponent, mask flags) [h][slot][c]: each half of a column
   // keeps its own copy, so no word crosses warps between barriers
   int *sword = P.scrW + (size_t)blockIdx.x * tile_slots * Geo<A>::H;
@@ -528,17 +607,20 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
     const int col = c_base + (valid ? cc0 : c_count - 1);
     const int32_t *alnc = P.aln + col;
     auto tok = [&](int n) { return __ldg(alnc + (size_t)n * C); };
-    auto slotv = [&](int s) { return svec + ((size_t)s * kTile + cl) * A + 32 * h; };
+    auto slotv = [&](int s) { return svec + (size_t)s * (kTile * A / 4); };
+    // this warp's rows of a branch's staging, and how many of them exist
+    const int cw0 = tile * kTile + 32 * (wk.warp & 3), nrows = c_count - cw0;
+    auto stage_row = [&](float *st, int n) { return st + ((size_t)(n - 1) * c_count + cw0) * A + 32 * h; };
     auto slotw = [&](int s) -> int & { return sword[(size_t)h * tile_slots + (size_t)s * kTile + cl]; };
     auto leaf = [&](BN<A> &o, int n) {
       const int t = tok(n);
       o.code = btcode(t, A);
-      wk.ld(o.cc, MT + ((size_t)n * (A + 1) + o.code) * A + 32 * h);
+      wk.ld_code(o.cc, MT + (size_t)n * (A + 1) * A + 32 * h, o.code);
       o.e = 0;
       o.hh = o.init = btung(t, A);
     };
     auto stored = [&](BN<A> &o, int s) {
-      wk.ld(o.cc, slotv(s));
+      wk.ld_slot(o.cc, slotv(s));
       const int w = slotw(s);
       o.e = w >> 2, o.hh = (w >> 1) & 1, o.init = w & 1, o.code = -1;
     };
@@ -593,7 +675,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
       } else {
         BV<A> cc;
         mprod(cc, u, s0.x, false);
-        wk.st(slotv(s0.y), cc);
+        wk.st_slot(slotv(s0.y), cc);
         slotw(s0.y) = (eU << 2) | (hh << 1) | init;
       }
     }
@@ -624,15 +706,14 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
                     const BV<A> *DM = nullptr) {
       float s = invP * __int_as_float((max(-127, min(127, eDU - eRoot)) + 127) << 23);
       s = active ? s : 0.f;
-      float *pa = stage_a + ((size_t)(n - 1) * c_count + (valid ? cc0 : c_count - 1)) * A + 32 * h;
-      float *pb = stage_b + ((size_t)(n - 1) * c_count + (valid ? cc0 : c_count - 1)) * A + 32 * h;
+      float *pa = stage_row(stage_a, n), *pb = stage_row(stage_b, n);
       if constexpr (MODE == 2 || MODE == 3) {
         BV<A> Ds;
 #pragma unroll
         for (int q = 0; q < S; ++q) Ds.v[q] = D.v[q] * s;
-        if ((MODE == 2 || stage_a) && valid) {
-          wk.st(pa, Ds);
-          wk.st(pb, U);
+        if (MODE == 2 || stage_a) {
+          wk.st_rows(pa, nrows, Ds);
+          wk.st_rows(pb, nrows, U);
         }
         if constexpr (MODE == 3) {
           // node posterior (D^T M_n) o U normalised over the states
@@ -689,11 +770,12 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
 #pragma unroll
         for (int q = 0; q < S; ++q) Ds.v[q] = D.v[q] * s;
         wk.matvec(dt, Ds, Vd, P.tab16 + (size_t)P.R * 24576);
-        if (leafcode >= 0) wk.ld(ut, Ut + leafcode * A + 32 * h);
-        else wk.matvec(ut, U, Vu, P.tab16 + (size_t)P.R * 24576 + 12288);
-        if (valid) {
-          wk.st(pa, dt);
-          wk.st(pb, ut);
+        wk.st_rows(pa, nrows, dt);
+        if (leafcode >= 0) {
+          wk.st_code(pb, nrows, Ut + 32 * h, leafcode);
+        } else {
+          wk.matvec(ut, U, Vu, P.tab16 + (size_t)P.R * 24576 + 12288);
+          wk.st_rows(pb, nrows, ut);
         }
       }
     };
@@ -704,14 +786,9 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
                        const uint16_t *MNg) {
       float s = invP * __int_as_float((max(-127, min(127, eDU - eRoot)) + 127) << 23);
       s = active ? s : 0.f;
-      float *pa = stage_a + ((size_t)(n - 1) * c_count + (valid ? cc0 : c_count - 1)) * A + 32 * h;
-      float *pb = stage_b + ((size_t)(n - 1) * c_count + (valid ? cc0 : c_count - 1)) * A + 32 * h;
-      wk.outside_tc(O, D, leafcode >= 0 ? nullptr : U, MNg, s, pa, pb, valid);
-      if (leafcode >= 0 && valid) {
-        BV<A> ut;
-        wk.ld(ut, Ut + leafcode * A + 32 * h);
-        wk.st(pb, ut);
-      }
+      float *pa = stage_row(stage_a, n), *pb = stage_row(stage_b, n);
+      wk.outside_tc(O, D, leafcode >= 0 ? nullptr : U, MNg, s, pa, pb, nrows);
+      if (leafcode >= 0) wk.st_code(pb, nrows, Ut + 32 * h, leafcode);
     };
     constexpr bool kFuse = TC && MODE == 1;
     auto act_of = [&](int n, int stn, int stpar) -> int {
@@ -743,7 +820,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
         stp = iRoot;
       } else {
         BV<A> D, U;
-        wk.ld(D, slotv(s0.y));
+        wk.ld_slot(D, slotv(s0.y));
         const int wd = slotw(s0.y);
         const int eD = wd >> 2;
         stp = (wd >> 1) & 1;
@@ -792,7 +869,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
           }
         } else if (ND || sc.y >= 0) {
           __syncwarp();
-          wk.st(slotv(sc.y), Dc);
+          wk.st_slot(slotv(sc.y), Dc);
           slotw(sc.y) = (eDc << 2) | (stc << 1) | actc;
         } else {
           const int gks[2] = {side ? s3.z : s3.x, side ? s3.w : s3.y};
@@ -841,7 +918,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
                 emit(gn[gs], Dg, U, g.code, eDg, actg);
               }
             } else {
-              wk.st(slotv(gks[gs]), Dg);
+              wk.st_slot(slotv(gks[gs]), Dg);
               slotw(gks[gs]) = (eDg << 2) | (stg << 1) | actg;
             }
           }
@@ -863,8 +940,8 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
 template <int A, int MODE, bool TC, bool F81M, bool ND>
 int walk_launch_nd(const KParams &p, float *sa, float *sb, int c_base, int c_count, int grid, cudaStream_t s) {
   const int threads = 128 * Geo<A>::H;
-  const size_t dyn = TC ? kTcDyn + 1024 : 0;
-  if (TC) {
+  const size_t dyn = (TC ? kTcDyn + 1024 : 0) + (Geo<A>::H == 2 ? 8 * kRowBuf : 0);
+  if (dyn) {
     cudaError_t e = cudaFuncSetAttribute(k_walk<A, MODE, TC, F81M, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)dyn);
     if (e != cudaSuccess) return (int)e;
