@@ -612,13 +612,26 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
     const int cw0 = tile * kTile + 32 * (wk.warp & 3), nrows = c_count - cw0;
     auto stage_row = [&](float *st, int n) { return st + ((size_t)(n - 1) * c_count + cw0) * A + 32 * h; };
     auto slotw = [&](int s) -> int & { return sword[(size_t)h * tile_slots + (size_t)s * kTile + cl]; };
-    auto leaf = [&](BN<A> &o, int n) {
-      const int t = tok(n);
+    // a step without derived nodes: its program entry and tokens, fetched a
+    // step ahead (the entry, the tokens and the leaf rows would otherwise wait
+    // for one another)
+    struct Step {
+      int p, sp, l, kl, r, kr, tp, tl, tr;
+      bool root;
+    };
+    auto step_prog = [&](Step &x, int i) {
+      const int4 s0 = __ldg(prog + 4 * i), s1 = __ldg(prog + 4 * i + 1), s2 = __ldg(prog + 4 * i + 2);
+      x.p = s0.x, x.sp = s0.y, x.root = s0.z != 0;
+      x.l = s1.x, x.kl = s1.y, x.r = s2.x, x.kr = s2.y;
+    };
+    auto step_tok = [&](Step &x) { x.tp = tok(x.p), x.tl = tok(x.l), x.tr = tok(x.r); };
+    auto leaf_tok = [&](BN<A> &o, int n, int t) {
       o.code = btcode(t, A);
       wk.ld_code(o.cc, MT + (size_t)n * (A + 1) * A + 32 * h, o.code);
       o.e = 0;
       o.hh = o.init = btung(t, A);
     };
+    auto leaf = [&](BN<A> &o, int n) { leaf_tok(o, n, tok(n)); };
     auto stored = [&](BN<A> &o, int s) {
       wk.ld_slot(o.cc, slotv(s));
       const int w = slotw(s);
@@ -650,22 +663,38 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
       wk.fill(ur, 1.f);
       wk.obs(ur, btcode(tok(0), A));
     }
+    Step cur;
+    if (ND && P.nsteps > 0) {
+      step_prog(cur, 0);
+      step_tok(cur);
+    }
     for (int i = 0; i < P.nsteps; ++i) {
-      const int4 s0 = prog[4 * i], s1 = prog[4 * i + 1], s2 = prog[4 * i + 2], s3 = prog[4 * i + 3];
+      int4 s0, s1, s2, s3{};
+      Step nxt;
+      if constexpr (ND) {
+        s0 = make_int4(cur.p, cur.sp, cur.root, 0);
+        s1 = make_int4(cur.l, cur.kl, 0, 0), s2 = make_int4(cur.r, cur.kr, 0, 0);
+        step_prog(nxt, min(i + 1, P.nsteps - 1));
+      } else {
+        s0 = prog[4 * i], s1 = prog[4 * i + 1], s2 = prog[4 * i + 2], s3 = prog[4 * i + 3];
+      }
       BN<A> nl, nr;
       {
         BV<A> u;
         BN<A> k0, k1;
         int cd;
         if (!ND && s1.y == -2) derive(nl, u, k0, k1, cd, s1.x, s1, s3.x, s3.y);
+        else if (ND && s1.y < 0) leaf_tok(nl, s1.x, cur.tl);
         else basic(nl, s1.x, s1.y);
         if (!ND && s2.y == -2) derive(nr, u, k0, k1, cd, s2.x, s2, s3.z, s3.w);
+        else if (ND && s2.y < 0) leaf_tok(nr, s2.x, cur.tr);
         else basic(nr, s2.x, s2.y);
+        if constexpr (ND) step_tok(nxt);
       }
       BV<A> u;
 #pragma unroll
       for (int q = 0; q < S; ++q) u.v[q] = nl.cc.v[q] * nr.cc.v[q];
-      wk.obs(u, btcode(tok(s0.x), A));
+      wk.obs(u, btcode(ND ? cur.tp : tok(s0.x), A));
       const int eU = nl.e + nr.e + wk.rescale(u);
       const int hh = nl.hh | nr.hh, init = nl.hh & nr.hh;
       if (s0.z) {
@@ -678,6 +707,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
         wk.st_slot(slotv(s0.y), cc);
         slotw(s0.y) = (eU << 2) | (hh << 1) | init;
       }
+      if constexpr (ND) cur = nxt;
     }
     // P = pi . U_root (combined over the pair)
     float pp = 0.f;
@@ -796,8 +826,20 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
       if (P.mask_mode == kMaskGiven) return P.mask[(size_t)n * C + col] != 0;
       return 1;
     };
+    if constexpr (ND) {
+      step_prog(cur, P.nsteps - 1);
+      step_tok(cur);
+    }
     for (int i = P.nsteps - 1; i >= 0; --i) {
-      const int4 s0 = prog[4 * i], s1 = prog[4 * i + 1], s2 = prog[4 * i + 2], s3 = prog[4 * i + 3];
+      int4 s0, s1, s2, s3{};
+      Step nxt;
+      if constexpr (ND) {
+        s0 = make_int4(cur.p, cur.sp, cur.root, 0);
+        s1 = make_int4(cur.l, cur.kl, 0, 0), s2 = make_int4(cur.r, cur.kr, 0, 0);
+        step_prog(nxt, max(i - 1, 0));
+      } else {
+        s0 = prog[4 * i], s1 = prog[4 * i + 1], s2 = prog[4 * i + 2], s3 = prog[4 * i + 3];
+      }
       BN<A> nl, nr;
       {
         // derived children's U and children are recomputed when they are
@@ -806,11 +848,14 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
         BN<A> k0, k1;
         int cd;
         if (!ND && s1.y == -2) derive(nl, u, k0, k1, cd, s1.x, s1, s3.x, s3.y);
+        else if (ND && s1.y < 0) leaf_tok(nl, s1.x, cur.tl);
         else basic(nl, s1.x, s1.y);
         if (!ND && s2.y == -2) derive(nr, u, k0, k1, cd, s2.x, s2, s3.z, s3.w);
+        else if (ND && s2.y < 0) leaf_tok(nr, s2.x, cur.tr);
         else basic(nr, s2.x, s2.y);
+        if constexpr (ND) step_tok(nxt);
       }
-      const int codep = btcode(tok(s0.x), A);
+      const int codep = btcode(ND ? cur.tp : tok(s0.x), A);
       BV<A> O;
       int eO, stp;
       if (s0.z) {
@@ -924,6 +969,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
           }
         }
       }
+      if constexpr (ND) cur = nxt;
     }
   }
   if constexpr (TC) {
