@@ -224,13 +224,19 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
                    : "memory");
     };
     if (t == 0)
-      for (int n = n_lo; n < n_lo + S - 1 && n < n_hi; ++n) load(n, it + (n - n_lo));
+      for (int n = n_lo; n < n_lo + S - 2 && n < n_hi; ++n) load(n, it + (n - n_lo));
     __syncwarp();
     float *scal = sm + Rg::SCAL;  // F81: piU, Dsum per column
     for (int n = n_lo; n < n_hi; ++n, ++it) {
-      // every thread is done with the stage of branch n - 1: refill it
-      __syncthreads();
-      if (t == 0 && n + S - 1 < n_hi) load(n + S - 1, it + S - 1);
+      // two branches per barrier: every thread is done with the stages of
+      // branches n - 2 and n - 1, refill them.  (F81: every branch, for the
+      // scalars)
+      const bool refill = ((n - n_lo) & 1) == 0;
+      if (F81 || refill) __syncthreads();
+      if (refill && t == 0) {
+        if (n + S - 2 < n_hi) load(n + S - 2, it + S - 2);
+        if (n + S - 1 < n_hi) load(n + S - 1, it + S - 1);
+      }
       __syncwarp();
       const int st = (int)(it % S);
       const float *cur = sm + st * Rg::STAGE;
