@@ -22,7 +22,6 @@
 // took 1245 us, most of it splitting and storing every branch's operands,
 // with 7e-7 of error against 2e-7 here.
 #include "common.cuh"
-#include "walk.cuh"
 
 namespace subby {
 namespace {
@@ -39,6 +38,20 @@ constexpr int kFRes = kFG * kFCol;
 constexpr size_t kFBytes = (size_t)(kFRes + kFS * kFStage) * sizeof(float);
 constexpr int kFT = 512;   // threads
 constexpr int kFBr = kFT / kFG;   // branches whose scalars and tokens are loaded together: one (branch, column) per thread
+
+constexpr int kWaitLimitT = 1 << 24;   // bounded mbarrier waits
+
+__device__ __forceinline__ bool mbar_wait_t(uint32_t mb, uint32_t phase) {
+  for (int it = 0; it < kWaitLimitT; ++it) {
+    uint32_t done;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(done)
+                 : "r"(mb), "r"(phase)
+                 : "memory");
+    if (done) return true;
+  }
+  return false;
+}
 
 __global__ void __launch_bounds__(kFT, 1)
     k_acc_f81(const KParams P, const float *__restrict__ sa, const float *__restrict__ sb,
@@ -121,7 +134,9 @@ __global__ void __launch_bounds__(kFT, 1)
     auto ahead = [&](int i0) {
       const int i = min(i0 + (t >> 3), nbr - 1), c = min(t & 7, gcols - 1);
       n_s = __ldg(sc + (size_t)i * c_count + g0 + c);
-      n_tok = __ldg(P.leaf + i + 1) ? btcode(__ldg(P.aln + (size_t)(i + 1) * C + c_base + g0 + c), kFA) : -1;
+      n_tok = __ldg(P.leaf + i + 1)
+                  ? (int)min((unsigned)__ldg(P.aln + (size_t)(i + 1) * C + c_base + g0 + c), (unsigned)kFA)
+                  : -1;
       if (t < kFBr) n_cf = __ldg(F8 + min(i0 + t, nbr - 1) + 1);
     };
     auto put = [&](int b) {
@@ -141,7 +156,7 @@ __global__ void __launch_bounds__(kFT, 1)
       }
       if (t < 32 && k + kFS - 1 < nst) load(k + kFS - 1);
       const uint32_t at = pos + k;
-      if (!mbar_wait((uint32_t)__cvta_generic_to_shared(&mbar[at % kFS]), (at / kFS) & 1)) s_err = 1;
+      if (!mbar_wait_t((uint32_t)__cvta_generic_to_shared(&mbar[at % kFS]), (at / kFS) & 1)) s_err = 1;
       const float *Ds = ring + (size_t)(at % kFS) * kFStage;
 #pragma unroll 2
       for (int x = 0; x < kFN; ++x) {
