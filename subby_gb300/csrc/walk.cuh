@@ -106,7 +106,7 @@ struct Walk {
   static constexpr int H = Geo<A>::H;
   static constexpr int S = Geo<A>::S;
   int c, h, warp, lane;
-  float4 *rows;   // H = 2: this warp's row buffer
+  float4 *rows;   // tensor-core walk: this warp's row buffer
   float *xch;     // shared exchange buffer: [2][32 states][128 cols] floats
   int *xmax;      // shared [2][128] ints (exponent-field exchange)
   TcState tcs;    // tensor-core state (per thread copy; used when use_tc)
@@ -296,9 +296,11 @@ struct Walk {
   }
   // The warp's columns as rows of A floats (p: row 0, this half's states),
   // nrows of them exist.  Written four rows of 128 bytes per instruction: a
-  // lane that stores its own row touches 32 lines with every 16 bytes.
+  // lane that stores its own row touches 32 lines with every 16 bytes.  (The
+  // FP32 products are bound by the load pipe, so that walk goes without the
+  // detour.)
   __device__ __forceinline__ void st_rows(float *p, int nrows, const BV<A> &x) const {
-    if constexpr (H == 2) {
+    if (H == 2 && use_tc) {
       __syncwarp();
 #pragma unroll
       for (int q = 0; q < 8; ++q)
@@ -316,7 +318,7 @@ struct Walk {
   }
   // row `code` of table T (this half's states) of every column of the warp
   __device__ __forceinline__ void ld_code(BV<A> &o, const float *T, int code) const {
-    if constexpr (H == 2) {
+    if (H == 2 && use_tc) {
       __syncwarp();
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
@@ -336,7 +338,7 @@ struct Walk {
   }
   // ... straight into the columns' rows at p
   __device__ __forceinline__ void st_code(float *p, int nrows, const float *T, int code) const {
-    if constexpr (H == 2) {
+    if (H == 2 && use_tc) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const int r = 4 * k + (lane >> 3), ch = lane & 7;
@@ -986,8 +988,8 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
 template <int A, int MODE, bool TC, bool F81M, bool ND>
 int walk_launch_nd(const KParams &p, float *sa, float *sb, int c_base, int c_count, int grid, cudaStream_t s) {
   const int threads = 128 * Geo<A>::H;
-  const size_t dyn = (TC ? kTcDyn + 1024 : 0) + (Geo<A>::H == 2 ? 8 * kRowBuf : 0);
-  if (dyn) {
+  const size_t dyn = TC ? kTcDyn + 1024 + 8 * kRowBuf : 0;
+  if (TC) {
     cudaError_t e = cudaFuncSetAttribute(k_walk<A, MODE, TC, F81M, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)dyn);
     if (e != cudaSuccess) return (int)e;
