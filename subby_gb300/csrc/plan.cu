@@ -1464,7 +1464,17 @@ int plan_pass4(subby_plan *P, int mode, bool post, int C, Launch &L) {
     while (L.block > 32 && bytes(L.block) > (size_t)maxsm) L.block -= 32;
     if (bytes(L.block) > (size_t)maxsm) return 1;
   }
-  while (L.block > 32 && C < P->nsm * L.block * L.columns) L.block = (L.block / 2 + 31) / 32 * 32;
+  if (per_sm == 1) {
+    // Large tables: waves of equal size.  A step's latency does not shrink
+    // with the CTA, so a few CTAs more than there are SMs cost a whole wave
+    // (R = 1023: 5000 columns in CTAs of 32 778 us, of 64 395 us; 20000
+    // columns in CTAs of 96 817 us, of 160 487 us).
+    const long long wave = (long long)P->nsm * L.block * L.columns, waves = (C + wave - 1) / wave;
+    const long long cols = waves * P->nsm * L.columns;
+    L.block = std::min(L.block, std::max(32, (int)((C + cols - 1) / cols + 31) / 32 * 32));
+  } else {
+    while (L.block > 32 && C < P->nsm * L.block * L.columns) L.block = (L.block / 2 + 31) / 32 * 32;
+  }
   L.smem = bytes(L.block);
   L.kernel = 5;
   L.small = false;

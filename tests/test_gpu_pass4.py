@@ -72,3 +72,11 @@ def test_trees(kind, leaves, C):
 def test_both_sides_of_two_columns_per_thread(extra):
     C = 384 * torch.cuda.get_device_properties(0).multi_processor_count + extra
     _check("random", 16, C, np.r_[0:70, C // 2:C // 2 + 70, C - 70:C], 7 + extra)
+
+
+# tables that leave one CTA per SM: whole warps per SM, and a column more
+@pytest.mark.parametrize("per_sm", [32, 33, 96])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_large_tables_in_equal_waves(per_sm, extra):
+    C = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    _check("random", 512, C, np.r_[0:8, C // 2:C // 2 + 8, C - 8:C], per_sm + extra, posteriors=False)
