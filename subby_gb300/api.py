@@ -174,13 +174,17 @@ class Plan:
             C = int(aln.shape[1])
             dev = aln.device
             res = {}
+            # (a buffer is only allocated when the caller brings none)
             out = out or {}
             if loglike:
-                res['logLike'] = out.get('logLike', torch.empty(C, dtype=torch.float32, device=dev))
+                res['logLike'] = out['logLike'] if 'logLike' in out else torch.empty(
+                    C, dtype=torch.float32, device=dev)
             if counts:
-                res['counts'] = out.get('counts', torch.empty((A, A, C), dtype=torch.float32, device=dev))
+                res['counts'] = out['counts'] if 'counts' in out else torch.empty(
+                    (A, A, C), dtype=torch.float32, device=dev)
             if rootprob:
-                res['rootProb'] = out.get('rootProb', torch.empty((A, C), dtype=torch.float32, device=dev))
+                res['rootProb'] = out['rootProb'] if 'rootProb' in out else torch.empty(
+                    (A, C), dtype=torch.float32, device=dev)
             dmask = None
             if mask_mode == _lib.MASK_GIVEN:
                 dmask = torch.as_tensor(np.asarray(mask) if not _is_torch(mask) else mask)
@@ -190,12 +194,12 @@ class Plan:
             stream = (stream if stream is not None else torch.cuda.current_stream(dev)).cuda_stream
 
             def dp(t):
-                return ct.c_void_p(t.data_ptr()) if t is not None else None
+                return t.data_ptr() if t is not None else None
             with self._lock, _device_ctx(dev):
                 _lib.check(lib.subby_plan_run(
-                    self._handle, dp(aln), C, dp(res.get('logLike')), dp(res.get('counts')),
+                    self._handle, aln.data_ptr(), C, dp(res.get('logLike')), dp(res.get('counts')),
                     dp(res.get('rootProb')), kind, mask_mode, dp(dmask),
-                    flags | _lib.DEVICE_PTRS, ct.c_void_p(stream)), "subby_plan_run")
+                    flags | _lib.DEVICE_PTRS, stream), "subby_plan_run")
             return res
         aln = _np(alignment, np.int32)
         if aln.ndim != 2 or aln.shape[0] != self.R:
@@ -385,6 +389,9 @@ class _device_ctx:
     def __enter__(self):
         if self.dev is not None:
             import torch
+            # nothing to switch (a device context costs more than the check)
+            if isinstance(self.dev, torch.device) and self.dev.index == torch.cuda.current_device():
+                return
             self.ctx = torch.cuda.device(self.dev)
             self.ctx.__enter__()
 
