@@ -13,7 +13,7 @@
 // and every matrix row, and Vd, Vu and pi are constant-bank operands.  The
 // tokens are read once: their codes travel in the words beside the vectors.
 // R = 255, 2^20 columns (GB300): 3227 -> 2097 us; R = 1023, 50001 columns
-// 1530 -> 545 us; node posteriors R = 127, 100001 columns 224 -> 132 us.
+// 1530 -> 549 us; node posteriors R = 127, 100001 columns 224 -> 132 us.
 // What bounds it: issue (60 %; 38 % of the instructions are integer work) and
 // the L2 / HBM latency of the node slots (294 MB for the resident columns,
 // 2.6 GB each way per 2^20 columns).  On the way there: without the codes in
