@@ -368,8 +368,8 @@ int subby_server_destroy(subby_server *server);
 int subby_debug_packed_queue_wait(int polls, int grid, int *gave_up);
 
 /* Test hook selecting the kernel so that every code path can be checked
- * against the oracle: 0 automatic (A = 4 tree kernel with tensor-memory
- * slots when it fits; A = 64 tree walk on the tensor cores), 1
+ * against the oracle: 0 automatic (the A = 4 kernels up to 1024 program
+ * steps; A = 64 tree walk on the tensor cores), 1
  * thread-per-column kernel (A <= 8) / warp-per-column kernel (larger A), 2
  * tree program with shared-memory slots (A <= 8) / FP32 CUDA-core tree walk
  * (larger A), 3 tree program with global-memory slots, 4 generic tree

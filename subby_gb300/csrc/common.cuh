@@ -114,7 +114,7 @@ struct KParams {
   const uint8_t *leaf;
   // k_pass4_packed: per step, the step of the internal child that waits on the stack
   const int *prog_other;
-  // branch joint posteriors (k_tree4, A = 4): (R, 4, 4, C) or the (4, 4, C)
+  // branch joint posteriors (k_pass4, A = 4): (R, 4, 4, C) or the (4, 4, C)
   // of node npost_node
   float *bpost;
   // irreversible models: complex tables (k_acccx.cu) and the choice of the

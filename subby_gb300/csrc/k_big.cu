@@ -230,7 +230,8 @@ __global__ void __launch_bounds__(256, 1) k_acc(const KParams P, const float *__
     for (int n = n_lo; n < n_hi; ++n, ++it) {
       // two branches per barrier: every thread is done with the stages of
       // branches n - 2 and n - 1, refill them.  (F81: every branch, for the
-      // scalars)
+      // scalars.)  A = 64, R = 127, 65536 columns 4.50 -> 4.41 ms, A = 20, R =
+      // 199, 20011 columns 312 -> 289 us against one branch per barrier.
       const bool refill = ((n - n_lo) & 1) == 0;
       if (F81 || refill) __syncthreads();
       if (refill && t == 0) {

@@ -512,7 +512,7 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
 
   // ---- tree program (k_tree, k_tree4): a node is DERIVED when both
   // children are leaves or stored (its CC is recomputed from them),
-  // otherwise STORED.  The walk (k_walk, slots in global memory) takes the
+  // otherwise STORED.  The walks (k_walk, k_qwalk, slots in global memory) take the
   // program in which every internal node is stored: a derived node costs
   // the walk one more M product (a tensor-core round trip at A = 64) in the
   // outside pass, a slot only 2 A floats per column.
