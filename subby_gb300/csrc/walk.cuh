@@ -25,9 +25,11 @@
 // its own column's 128-byte row touches 32 lines per 16-byte instruction, so
 // slot vectors are lane-interleaved, and leaf rows and staged rows move four
 // whole rows per instruction through a per-warp buffer; the next step's
-// program entry and tokens are fetched a step ahead.  Counts walk of R = 127,
-// 65536 columns (GB300): 5.24 ms, 3.85 ms with the rows, 3.60 ms with both
-// (load pipe 54 -> 26 %).
+// program entry and tokens are fetched a step ahead, a product's matrix is
+// requested before the step's loads, and a step's leaf products are read in
+// the next step.  Counts walk of R = 127, 65536 columns (GB300): 5.24 ms; 3.85
+// ms with the rows (load pipe 54 -> 26 %), 3.60 ms with the tokens, 3.39 ms
+// with the matrices and the leaves.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -234,10 +236,11 @@ struct Walk {
   // two-term split measured 1.5e-4 column-wise counts error at A = 64).
   // Bg: the B tile's three terms (4096 elements each) in the canonical
   // layout in global memory, brought in by bulk copies.
-  __device__ __forceinline__ void matvec_tc(BV<A> &y, const BV<A> &x, const uint16_t *Bg) {
+  // (loaded: the caller has issued load_node_B already.)
+  __device__ __forceinline__ void matvec_tc(BV<A> &y, const BV<A> &x, const uint16_t *Bg, bool loaded = false) {
     static_assert(A == 64, "tensor-core walk is A = 64");
     TcState &T = tcs;
-    load_node_B(Bg);
+    if (!loaded) load_node_B(Bg);
     stage_x(x, T.sA);
     tc_sync();
     if (threadIdx.x == 0) {
@@ -257,10 +260,10 @@ struct Walk {
   //   MNg is given, dt alone (N = 64) otherwise; ut = Vu-product of U when U
   //   is given.  dt is scaled by s and stored to pa, ut to pb (st_rows).
   __device__ __forceinline__ void outside_tc(BV<A> &O, const BV<A> &D, const BV<A> *U, const uint16_t *MNg,
-                                             float s, float *pa, float *pb, int nrows) {
+                                             float s, float *pa, float *pb, int nrows, bool loaded = false) {
     TcState &T = tcs;
     const bool wantO = MNg != nullptr, wantU = U != nullptr;
-    if (wantO) load_node_B(MNg);
+    if (wantO && !loaded) load_node_B(MNg);
     stage_x(D, T.sA);
     if (wantU) stage_x(*U, T.sA + kSA1);
     tc_sync();
@@ -291,6 +294,28 @@ struct Walk {
       st_rows(pb, nrows, t);
     }
     if (wantO) tm_ld32(O, 32u * h);
+  }
+
+  // The Vd products of a step's leaf branches, left in operand 0 to the dt
+  // columns and right in operand 1 to the ut columns: issued here, read by
+  // leaf_read after an mma_wait.
+  __device__ __forceinline__ void leaf_issue(bool left, bool right) {
+    TcState &T = tcs;
+    tc_sync();
+    if (threadIdx.x == 0) {
+      if (left) mma6(T.tmem + 64, T.sA, 16384, T.sA + kSB2 + 8192, 16384, kIdesc);
+      if (right) mma6(T.tmem + 128, T.sA + kSA1, 16384, T.sA + kSB2 + 8192, 16384, kIdesc);
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(T.mbM)
+                   : "memory");
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ void leaf_read(bool right, float s, float *pa, int nrows) {
+    BV<A> t;
+    tm_ld32(t, (right ? 128u : 64u) + 32u * h);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) t.v[i] *= s;
+    st_rows(pa, nrows, t);
   }
 
   __device__ __forceinline__ void ld(BV<A> &o, const float *p) const {  // S contiguous floats
@@ -670,6 +695,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
     };
 
     // ---------------------------------------------------------------- inside
+    constexpr bool kEarlyB = TC && MODE == 1 && ND && !f81m;
     BV<A> ur;
     int eRoot = 0, iRoot = 0;
     if (P.root_is_leaf) {
@@ -688,6 +714,11 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
         s0 = make_int4(cur.p, cur.sp, cur.root, 0);
         s1 = make_int4(cur.l, cur.kl, 0, 0), s2 = make_int4(cur.r, cur.kr, 0, 0);
         step_prog(nxt, min(i + 1, P.nsteps - 1));
+        // the product's matrix arrives under the step's loads (its place is
+        // free: the last product was waited for)
+        if constexpr (kEarlyB) {
+          if (!cur.root) wk.load_node_B(P.tab16 + (size_t)cur.p * 24576);
+        }
       } else {
         s0 = prog[4 * i], s1 = prog[4 * i + 1], s2 = prog[4 * i + 2], s3 = prog[4 * i + 3];
       }
@@ -716,7 +747,8 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
         iRoot = init;
       } else {
         BV<A> cc;
-        mprod(cc, u, s0.x, false);
+        if constexpr (kEarlyB) wk.matvec_tc(cc, u, P.tab16 + (size_t)s0.x * 24576, true);
+        else mprod(cc, u, s0.x, false);
         wk.st_slot(slotv(s0.y), cc);
         slotw(s0.y) = (eU << 2) | (hh << 1) | init;
       }
@@ -826,14 +858,26 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
     // trip (Walk::outside_tc); O receives the MN product when MNg is given
     BV<A> Onone;
     auto emit_tc = [&](int n, const BV<A> &D, const BV<A> *U, int leafcode, int eDU, int active, BV<A> &O,
-                       const uint16_t *MNg) {
+                       const uint16_t *MNg, bool loaded = false) {
       float s = invP * __int_as_float((max(-127, min(127, eDU - eRoot)) + 127) << 23);
       s = active ? s : 0.f;
       float *pa = stage_row(stage_a, n), *pb = stage_row(stage_b, n);
-      wk.outside_tc(O, D, leafcode >= 0 ? nullptr : U, MNg, s, pa, pb, nrows);
+      wk.outside_tc(O, D, leafcode >= 0 ? nullptr : U, MNg, s, pa, pb, nrows, loaded);
       if (leafcode >= 0) wk.st_code(pb, nrows, Ut + 32 * h, leafcode);
     };
     constexpr bool kFuse = TC && MODE == 1;
+    // Leaf branches of the derived-node-free instance: a step's products are
+    // issued together and read in the next step, after its loads.
+    bool pend_l = false, pend_r = false;
+    int pend_nl = 0, pend_nr = 0;
+    float pend_sl = 0.f, pend_sr = 0.f;
+    auto flush = [&]() {
+      if (!pend_l && !pend_r) return;
+      wk.mma_wait();
+      if (pend_l) wk.leaf_read(false, pend_sl, stage_row(stage_a, pend_nl), nrows);
+      if (pend_r) wk.leaf_read(true, pend_sr, stage_row(stage_a, pend_nr), nrows);
+      pend_l = pend_r = false;
+    };
     auto act_of = [&](int n, int stn, int stpar) -> int {
       if (P.mask_mode == kMaskAuto) return stn & stpar;
       if (P.mask_mode == kMaskGiven) return P.mask[(size_t)n * C + col] != 0;
@@ -850,6 +894,9 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
         s0 = make_int4(cur.p, cur.sp, cur.root, 0);
         s1 = make_int4(cur.l, cur.kl, 0, 0), s2 = make_int4(cur.r, cur.kr, 0, 0);
         step_prog(nxt, max(i - 1, 0));
+        if constexpr (kEarlyB) {
+          if (!cur.root) wk.load_node_B(P.tab16 + (size_t)cur.p * 24576 + 12288);
+        }
       } else {
         s0 = prog[4 * i], s1 = prog[4 * i + 1], s2 = prog[4 * i + 2], s3 = prog[4 * i + 3];
       }
@@ -892,7 +939,8 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
             mprod(O, D, s0.x, true);
             emit_tc(s0.x, D, &U, -1, eD + eUp, actp, Onone, nullptr);
           } else {
-            emit_tc(s0.x, D, &U, -1, eD + eUp, actp, O, P.tab16 + (size_t)s0.x * 24576 + 12288);
+            if constexpr (kEarlyB) flush();
+            emit_tc(s0.x, D, &U, -1, eD + eUp, actp, O, P.tab16 + (size_t)s0.x * 24576 + 12288, kEarlyB);
           }
         } else if constexpr (MODE == 3) {
           mprod(O, D, s0.x, true);
@@ -917,7 +965,12 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
         const int stc = me.init | (stp & me.hh);
         const int actc = act_of(sc.x, stc, stp);
         if (sc.y == -1) {
-          if constexpr (kFuse) {
+          if constexpr (kEarlyB) {
+            const float sw = invP * __int_as_float((max(-127, min(127, eDc - eRoot)) + 127) << 23);
+            wk.stage_x(Dc, wk.tcs.sA + (side ? kSA1 : 0u));
+            if (side) pend_r = true, pend_nr = sc.x, pend_sr = actc ? sw : 0.f;
+            else pend_l = true, pend_nl = sc.x, pend_sl = actc ? sw : 0.f;
+          } else if constexpr (kFuse) {
             emit_tc(sc.x, Dc, nullptr, me.code, eDc, actc, Onone, nullptr);
           } else {
             BV<A> U;
@@ -982,8 +1035,16 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
           }
         }
       }
+      if constexpr (kEarlyB) {
+        if (pend_l || pend_r) {
+          wk.leaf_issue(pend_l, pend_r);
+          if (pend_l) wk.st_code(stage_row(stage_b, s1.x), nrows, Ut + 32 * h, nl.code);
+          if (pend_r) wk.st_code(stage_row(stage_b, s2.x), nrows, Ut + 32 * h, nr.code);
+        }
+      }
       if constexpr (ND) cur = nxt;
     }
+    if constexpr (kEarlyB) flush();
   }
   if constexpr (TC) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
