@@ -10,7 +10,8 @@
 // for the representatives k only (a real l has no partner: J_kl' = 0), and
 //   counts_ij = sum_k w_k Re(V_ik (C Vinv)_kj), w = 2 for a pair, 1 for a real
 // (off the diagonal times Q_ij).  That is half the complex products of the
-// full C.  Plans whose eigensystem does not pair up keep k_acc_cx.
+// full C.  Plans whose eigensystem does not pair up, or is ill-conditioned (kCxCond),
+// keep k_acc_cx.
 //
 // k_acc_cx forms a column's D~, U~ one dot product per thread from strided
 // rows and shares no load between columns.  Here k_projx projects with the

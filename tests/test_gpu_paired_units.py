@@ -1,7 +1,9 @@
 """Irreversible counts over conjugate-paired units (k_projx, k_accx) at A =
 16, 20, 32 against the FP64 oracle: eigensystems with pairs and reals, with
-reals only (a reversible matrix in irreversible form) and one that is not in
-conjugate form (its columns carry phases: the general kernel); one column, a
+reals only (a reversible matrix in irreversible form), pairs with orthogonal
+eigenvectors (a circulant matrix; the random ones are often too ill-conditioned
+at A = 32 for the units) and one that is not in conjugate form (its columns
+carry phases: the general kernel); one column, a
 block of columns and one more, more branches than one run of the register
 sums.  Tolerance: the irreversible bar, 1e-4 x max(1, cond(V) / 10)."""
 import numpy as np
@@ -25,6 +27,12 @@ def _model(A, kind, rng):
     if kind == "reals":
         _, log_exch, pi = models.random_reversible(A, rng, 0.5, 2.0)
         return models.irrev_model_from_rate_matrix(models.reversible_rate_matrix(log_exch, pi), pi)
+    if kind == "circulant":
+        r = rng.gamma(1.0, size=A)
+        r[0] = 0.0
+        Q = np.stack([np.roll(r, i) for i in range(A)]) / r.sum()
+        np.fill_diagonal(Q, -1.0)
+        return models.irrev_model_from_rate_matrix(Q, np.full(A, 1.0 / A))
     m = models.random_irreversible(A, rng)
     if kind == "phases":
         f = np.exp(1j * rng.uniform(0, 2 * np.pi, A)) * rng.uniform(0.5, 2.0, A)
@@ -33,7 +41,7 @@ def _model(A, kind, rng):
 
 
 @pytest.mark.parametrize("A", [16, 20, 32])
-@pytest.mark.parametrize("kind", ["pairs", "reals", "phases"])
+@pytest.mark.parametrize("kind", ["pairs", "reals", "circulant", "phases"])
 @pytest.mark.parametrize("leaves,C", [(2, 1), (9, 129), (40, 57)])
 def test_counts(A, kind, leaves, C):
     rng = np.random.default_rng(A + leaves)
