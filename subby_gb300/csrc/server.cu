@@ -9,7 +9,8 @@
 //    descriptors (the engine copies the tree and model) and collect
 //    completions; nothing on their side touches CUDA;
 //  * prepared plans (tree program, M(t), J(t) and operand tables) stay
-//    resident in an LRU cache keyed by a hash of tree and model;
+//    resident in an LRU cache keyed by a hash of tree and model, pinned
+//    while a run uses them (plan_cache.h);
 //  * short A = 4 jobs waiting together run as one launch of the persistent
 //    packed kernel over their flattened (job, 256-column tile) queue
 //    (k_pass4_packed);
@@ -42,7 +43,6 @@
 #include <condition_variable>
 #include <cstring>
 #include <deque>
-#include <list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -51,6 +51,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "plan_cache.h"
 #include "subby_gb300.h"
 
 namespace subby {
@@ -164,11 +165,7 @@ struct Run {
   size_t bytes = 0;
 };
 
-struct PlanEntry {
-  subby_plan *p = nullptr;
-  bool busy = false;
-  std::list<uint64_t>::iterator lru;
-};
+using Plans = subby::PlanCache<subby_plan *, int (*)(subby_plan *)>;
 
 struct Slot {
   cudaStream_t s_norm = nullptr, s_hi = nullptr;
@@ -202,8 +199,7 @@ struct subby_server {
 
   std::vector<Slot> slots;
   std::vector<int> free_slots;
-  std::unordered_map<uint64_t, PlanEntry> plans;
-  std::list<uint64_t> lru;
+  Plans plans{subby_plan_destroy};
   PinnedPool pinned;
 
   std::mutex mu;                      // submissions, completions, release
@@ -256,43 +252,23 @@ size_t job_bytes(int R, int C, int A) {
 
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
+// The job's plan, pinned: a run's plans stay until its completion drops
+// them, whatever else is prepared meanwhile (the other jobs of its batch).
 int plan_for(subby_server *S, SJob *j, subby_plan **out) {
-  auto it = S->plans.find(j->key);
-  if (it != S->plans.end()) {
-    S->lru.erase(it->second.lru);
-    S->lru.push_front(j->key);
-    it->second.lru = S->lru.begin();
-    *out = it->second.p;
-    return SUBBY_OK;
-  }
+  if ((*out = S->plans.take(j->key))) return SUBBY_OK;
   subby_plan *p = nullptr;
   const int rc = subby_plan_create(j->parent.data(), j->dist.data(), j->ev.data(), j->V.data(), j->pi.data(),
                                    j->d.R, j->d.A, &p);
   if (rc != 0) return rc;
-  S->lru.push_front(j->key);
-  S->plans[j->key] = PlanEntry{p, false, S->lru.begin()};
-  // evict least recently used plans that no job is running
-  while ((int)S->plans.size() > S->plan_cache) {
-    bool evicted = false;
-    for (auto r = S->lru.rbegin(); r != S->lru.rend(); ++r) {
-      auto e = S->plans.find(*r);
-      if (e != S->plans.end() && !e->second.busy && e->first != j->key) {
-        subby_plan_destroy(e->second.p);
-        S->lru.erase(std::next(r).base());
-        S->plans.erase(e);
-        evicted = true;
-        break;
-      }
-    }
-    if (!evicted) break;
-  }
+  S->plans.add(j->key, p, S->plan_cache);
   *out = p;
   return SUBBY_OK;
 }
 
-bool plan_busy(subby_server *S, uint64_t key) {
-  auto it = S->plans.find(key);
-  return it != S->plans.end() && it->second.busy;
+// A run of several jobs is over, or one that was not started.
+void drop_plans(subby_server *S, const std::vector<SJob *> &jobs) {
+  for (SJob *j : jobs) S->plans.drop(j->key);
+  S->plans.trim(S->plan_cache);
 }
 
 bool fits(subby_server *S, SJob *j) {
@@ -303,7 +279,7 @@ bool fits(subby_server *S, SJob *j) {
       for (SJob *k : r->jobs) longs += k->cost_ms > S->short_ms;
     if (longs >= S->max_inflight - S->short_slots) return false;
   }
-  if (plan_busy(S, j->key)) return false;
+  if (S->plans.pinned(j->key)) return false;
   return S->used + j->bytes <= S->budget || S->inflight.empty();
 }
 
@@ -324,13 +300,13 @@ int grow_arena(subby_server *S, Slot &sl, size_t need, cudaStream_t s) {
   return 0;
 }
 
+// (the jobs' plans are pinned)
 void start_run(subby_server *S, int slot_i, const std::vector<SJob *> &jobs) {
   Slot &sl = S->slots[slot_i];
   S->free_slots.erase(std::find(S->free_slots.begin(), S->free_slots.end(), slot_i));
   Run *run = new Run();
   run->slot = slot_i;
   for (SJob *j : jobs) {
-    S->plans[j->key].busy = true;
     j->slot = slot_i;
     run->jobs.push_back(j);
     run->bytes += j->bytes;
@@ -358,6 +334,7 @@ int launch(subby_server *S, SJob *j) {
   auto bail = [&](int rc) {
     cudaStreamSynchronize(st);
     cudaGetLastError();
+    drop_plans(S, {j});
     return rc;
   };
   const bool wl = d.want & SUBBY_WANT_LOGLIKE, wc = d.want & SUBBY_WANT_COUNTS, wr = d.want & SUBBY_WANT_ROOTPROB;
@@ -437,9 +414,11 @@ int launch_batch(subby_server *S, std::vector<SJob *> &batch) {
   const int slot_i = S->free_slots.back();
   Slot &sl = S->slots[slot_i];
   cudaStream_t st = sl.s_hi;
+  std::vector<SJob *> held;   // jobs whose plans this batch has pinned and not handed to a run
   auto bail = [&](int rc) {
     cudaStreamSynchronize(st);
     cudaGetLastError();
+    drop_plans(S, held);
     return rc;
   };
   const bool counts = batch[0]->d.want & SUBBY_WANT_COUNTS;
@@ -449,7 +428,8 @@ int launch_batch(subby_server *S, std::vector<SJob *> &batch) {
   std::vector<subby_plan *> plans(n, nullptr);
   for (int i = 0; i < n; ++i) {
     const int rc = plan_for(S, batch[i], &plans[i]);
-    if (rc) return rc;
+    if (rc) return bail(rc);
+    held.push_back(batch[i]);
   }
   // device layout: per job tokens and outputs, then the queue
   std::vector<size_t> o_tok(n), o_out(n);
@@ -536,7 +516,10 @@ int launch_batch(subby_server *S, std::vector<SJob *> &batch) {
     taken_plans.push_back(plans[i]);
     ++njobs;
   }
-  if (njobs == 0) return 0;
+  if (njobs == 0) {
+    drop_plans(S, held);
+    return 0;
+  }
   hq[0] = 0;          // head
   hq[1] = (int)nit;   // published: every item
   hq[2] = 1;          // closed
@@ -564,6 +547,8 @@ int launch_batch(subby_server *S, std::vector<SJob *> &batch) {
       cudaEventRecord(sl.done, st) != cudaSuccess)
     return bail(SUBBY_ERR_CUDA);
   start_run(S, slot_i, taken);
+  held.erase(std::remove_if(held.begin(), held.end(), [](SJob *j) { return !j->nopack; }), held.end());
+  drop_plans(S, held);   // the jobs left out
   S->packed_jobs += njobs;
   S->packed_launches += 1;
   return njobs;
@@ -609,7 +594,7 @@ void engine(subby_server *S) {
       long long cols = 0;
       size_t bytes = 0;
       for (SJob *w : S->waiting) {
-        if (!packable(S, w) || plan_busy(S, w->key) || (!cand.empty() && !same_group(cand[0], w))) continue;
+        if (!packable(S, w) || S->plans.pinned(w->key) || (!cand.empty() && !same_group(cand[0], w))) continue;
         if (S->used + bytes + w->bytes > S->budget && !(S->inflight.empty() && cand.empty())) continue;
         cand.push_back(w);
         cols += w->d.C;
@@ -676,13 +661,11 @@ void engine(subby_server *S) {
         status = SUBBY_ERR_TIMEOUT;
       }
       for (SJob *j : r->jobs) {
-        auto it = S->plans.find(j->key);
-        if (it != S->plans.end()) {
-          it->second.busy = false;
-          if (r->jobs.size() == 1) subby_plan_trim(it->second.p);  // workspace back to the pool, in stream order
-        }
-        finish(S, j, status);
+        subby_plan *p = S->plans.drop(j->key);
+        if (p && r->jobs.size() == 1) subby_plan_trim(p);  // workspace back to the pool, in stream order
       }
+      S->plans.trim(S->plan_cache);
+      for (SJob *j : r->jobs) finish(S, j, status);
       sl.run = nullptr;
       S->free_slots.push_back(r->slot);
       S->used -= r->bytes;
@@ -896,7 +879,7 @@ int subby_server_destroy(subby_server *S) {
   }
   cudaSetDevice(S->device);
   cudaDeviceSynchronize();
-  for (auto &kv : S->plans) subby_plan_destroy(kv.second.p);
+  S->plans.clear();
   for (auto &kv : S->held) delete kv.second;
   for (SJob *j : S->completed) delete j;
   for (Slot &sl : S->slots) {
