@@ -209,15 +209,11 @@ cudaError_t pool_alloc(void **p, size_t bytes, cudaMemPool_t pool, cudaStream_t 
 struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
-  // Grow to `need` bytes in stream order on `s`; the old block is freed on
-  // `s` once `after` (the plan's last use, possibly on another stream) has
-  // completed.
-  int grow(size_t need, cudaStream_t s, cudaMemPool_t pool, cudaEvent_t after) {
+  // Grow to `need` bytes in stream order on `s`, which comes after every
+  // enqueued use of the old block.
+  int grow(size_t need, cudaStream_t s, cudaMemPool_t pool) {
     if (need <= bytes) return 0;
-    if (p) {
-      if (after) cudaStreamWaitEvent(s, after, 0);
-      cudaFreeAsync(p, s);
-    }
+    if (p) cudaFreeAsync(p, s);
     p = nullptr;
     bytes = 0;
     size_t want = need + need / 4;
@@ -299,15 +295,39 @@ struct subby_plan {
   DevBuf io;       // staging of alignment/mask/outputs in host-pointer mode
   // host-pointer mode: copy queues of the column-chunk pipeline and its events
   cudaStream_t s_in = nullptr, s_out = nullptr;
-  // stream-ordered lifetime: tables are built on s_prep; last_use marks the
-  // end of the latest enqueued kernel, after which buffers may be freed
+  // Stream order.  Tables are built on s_prep (`ready`: their end there) and
+  // buffers are freed on it, after the enqueued runs: `use` marks the end of
+  // the latest run that reads tables only, `work_use` that of the latest one
+  // that also writes `work`.  Runs of the first kind overlap freely on
+  // different streams, so s_prep collects their marks; a run of the second
+  // kind on another stream waits for the one before it, whose scratch it
+  // takes over.
+  struct Mark {
+    cudaEvent_t e = nullptr;
+    bool set = false;
+    unsigned long long stream = 0;   // its stream's id (unique; a handle may be that of a destroyed stream)
+  };
   cudaStream_t s_prep = nullptr;
-  cudaEvent_t last_use = nullptr;
-  cudaEvent_t ready = nullptr;   // end of the table preparation on s_prep
-  bool used = false;
+  cudaEvent_t ready = nullptr;
+  Mark use, work_use;
   cudaMemPool_t pool = nullptr;
-  int grow(DevBuf &b, size_t need, cudaStream_t s) {
-    return b.grow(need, s, pool, used ? last_use : nullptr);
+  // `s` after every enqueued run
+  cudaError_t wait_runs(cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    for (const Mark *m : {&use, &work_use})
+      if (e == cudaSuccess && m->set) e = cudaStreamWaitEvent(s, m->e, 0);
+    return e;
+  }
+  // `s` after the latest use of `work`, which then holds `need` bytes
+  int grow_work(size_t need, cudaStream_t s) {
+    unsigned long long id = 0;
+    cudaError_t e = cudaStreamGetId(s, &id);
+    if (e == cudaSuccess && work_use.set && work_use.stream != id) e = cudaStreamWaitEvent(s, work_use.e, 0);
+    return e == cudaSuccess ? work.grow(need, s, pool) : cuda_fail(e, "workspace order");
+  }
+  int grow_io(size_t need, cudaStream_t s) {
+    if (need > io.bytes) wait_runs(s);
+    return io.grow(need, s, pool);
   }
   std::vector<cudaEvent_t> ev;
   std::mutex lock;
@@ -509,7 +529,8 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
     int lo = 0, hi = 0;
     cudaDeviceGetStreamPriorityRange(&lo, &hi);
     cudaError_t e0 = cudaStreamCreateWithPriority(&P->s_prep, cudaStreamNonBlocking, hi);
-    if (e0 == cudaSuccess) e0 = cudaEventCreateWithFlags(&P->last_use, cudaEventDisableTiming);
+    if (e0 == cudaSuccess) e0 = cudaEventCreateWithFlags(&P->use.e, cudaEventDisableTiming);
+    if (e0 == cudaSuccess) e0 = cudaEventCreateWithFlags(&P->work_use.e, cudaEventDisableTiming);
     if (e0 == cudaSuccess) e0 = cudaEventCreateWithFlags(&P->ready, cudaEventDisableTiming);
     if (e0 != cudaSuccess) {
       subby_plan_destroy(P);
@@ -1140,7 +1161,7 @@ int subby_plan_destroy(subby_plan *P) {
   // frees are ordered after the plan's last enqueued kernel; nothing here
   // waits for the device
   cudaStream_t s = P->s_prep;
-  if (s && P->used) cudaStreamWaitEvent(s, P->last_use, 0);
+  if (s) P->wait_runs(s);
   if (P->s_in) cudaStreamSynchronize(P->s_in);
   if (P->s_out) cudaStreamSynchronize(P->s_out);
   void *bufs[] = {P->d_tab, P->d_tab64, P->d_steps, P->d_slots, P->d_prog, P->d_prog_w, P->d_prog_s, P->d_prog_i, P->d_prog_other, P->d_leaf, P->d_cxu, P->d_tab16, P->d_err,
@@ -1150,7 +1171,8 @@ int subby_plan_destroy(subby_plan *P) {
   P->work.release(s);
   P->io.release(s);
   for (cudaEvent_t e : P->ev) cudaEventDestroy(e);
-  if (P->last_use) cudaEventDestroy(P->last_use);
+  for (auto *m : {&P->use, &P->work_use})
+    if (m->e) cudaEventDestroy(m->e);
   if (P->ready) cudaEventDestroy(P->ready);
   if (P->s_in) cudaStreamDestroy(P->s_in);
   if (P->s_out) cudaStreamDestroy(P->s_out);
@@ -1168,8 +1190,7 @@ int subby_plan_status(subby_plan *P) {
   cudaGetDevice(&cur);
   if (cur != P->device) cudaSetDevice(P->device);
   int dev_err = 0;
-  cudaError_t e = cudaSuccess;
-  if (P->used) e = cudaStreamWaitEvent(P->s_prep, P->last_use, 0);
+  cudaError_t e = P->wait_runs(P->s_prep);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&dev_err, P->d_err, sizeof(int), cudaMemcpyDeviceToHost, P->s_prep);
   if (e == cudaSuccess) e = cudaStreamSynchronize(P->s_prep);
   if (e == cudaSuccess && dev_err) {
@@ -1198,7 +1219,7 @@ int subby_plan_set_root_prior(subby_plan *P, const double *root_prior) {
   cudaGetDevice(&cur);
   if (cur != P->device) cudaSetDevice(P->device);
   // after every enqueued use of the tables; later runs wait for `ready`
-  cudaError_t e = P->used ? cudaStreamWaitEvent(P->s_prep, P->last_use, 0) : cudaSuccess;
+  cudaError_t e = P->wait_runs(P->s_prep);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(P->d_tab + P->off.pi0, h.data(), sizeof(float) * A, cudaMemcpyHostToDevice, P->s_prep);
   if (e == cudaSuccess) e = cudaEventRecord(P->ready, P->s_prep);
@@ -1214,7 +1235,7 @@ int subby_plan_trim(subby_plan *P) {
   int cur = 0;
   cudaGetDevice(&cur);
   if (cur != P->device) cudaSetDevice(P->device);
-  if (P->used) cudaStreamWaitEvent(P->s_prep, P->last_use, 0);
+  P->wait_runs(P->s_prep);
   P->work.release(P->s_prep);
   P->io.release(P->s_prep);
   if (cur != P->device) cudaSetDevice(cur);
@@ -1536,11 +1557,17 @@ int plan_pass4(subby_plan *P, int mode, bool post, int C, Launch &L) {
 // staging (2 (R-1) A floats per column) stays within kStageBudget bytes.
 constexpr size_t kStageBudget = size_t(4) << 30;
 
-// Marks the end of the work just enqueued on `stream` as the plan's last use.
-int mark_use(subby_plan *P, cudaStream_t stream) {
-  CU(cudaEventRecord(P->last_use, stream));
-  P->used = true;
-  return 0;
+// The end, on `stream`, of a run (work: one that used P->work).
+int mark_use(subby_plan *P, cudaStream_t stream, bool work) {
+  subby_plan::Mark &m = work ? P->work_use : P->use;
+  unsigned long long id = 0;
+  CU(cudaStreamGetId(stream, &id));
+  // the mark moves to another stream: frees stay after the run that it leaves
+  if (!work && m.set && m.stream != id) CU(cudaStreamWaitEvent(P->s_prep, m.e, 0));
+  CU(cudaEventRecord(m.e, stream));
+  m.set = true;
+  m.stream = id;
+  return SUBBY_OK;
 }
 
 // Parameters of the walk (k_walk) and the kernels that consume its staging.
@@ -1658,7 +1685,7 @@ int run_big(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_
   // A = 64 F81 counts (k_acc_f81): per-branch scalars staged too
   const bool f81_64 = A == 64 && counts && (mode & kModeF81) && !(mode & kModeBranch);
   const size_t stage_c_bytes = f81_64 ? al256((size_t)(R - 1) * chunk * sizeof(float2)) : 0;
-  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * stage_bytes + stage_c_bytes + 256, stream))) return rc;
+  if ((rc = P->grow_work(w.vec_bytes + w.word_bytes + 2 * stage_bytes + stage_c_bytes + 256, stream))) return rc;
   char *base = place_walk(k, w, P->work.p);
   float *sa = (float *)base;
   float *sb = (float *)(base + stage_bytes);
@@ -1687,7 +1714,7 @@ int run_big(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_
       g_launches += 1;
     }
   }
-  return mark_use(P, stream);
+  return mark_use(P, stream, true);
 }
 
 // Node / branch posteriors.  The walk (mode 3) writes the node posteriors of
@@ -1702,7 +1729,7 @@ int run_post(subby_plan *P, const int32_t *d_aln, int C, int node, float *d_node
   const bool all = node < 0;
   if (all && d_br) CU(cudaMemsetAsync(d_br, 0, (size_t)A * A * C * sizeof(float), stream));
   const bool outside = R > 1 && node != 0;
-  if (!outside && !d_node) return mark_use(P, stream);
+  if (!outside && !d_node) return mark_use(P, stream, false);
   if (A == 4 && R > 1) {
     // directly from the A = 4 kernels: the root alone without an outside pass
     Launch L4;
@@ -1733,7 +1760,7 @@ int run_post(subby_plan *P, const int32_t *d_aln, int C, int node, float *d_node
       } else {
         const size_t n4 = (size_t)k.nsteps * L4.columns * L4.nworkers;
         int rc;
-        if ((rc = P->grow(P->work, al256(n4 * 16) + n4 * 4 + 256, stream))) return rc;
+        if ((rc = P->grow_work(al256(n4 * 16) + n4 * 4 + 256, stream))) return rc;
         k.scrV = (float *)P->work.p;
         k.scrW = (int *)((char *)P->work.p + al256(n4 * 16));
         lr = launch_pass4(k, P->prog_i.data(), P->prog_other.data(), P->hVd.data(), P->hVu.data(), P->hpi, false, kMaskNone, true, L4.columns, L4.grid,
@@ -1741,7 +1768,7 @@ int run_post(subby_plan *P, const int32_t *d_aln, int C, int node, float *d_node
       }
       if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("kernel launch failed: ") + cudaGetErrorString((cudaError_t)lr));
       g_launches += 1;
-      return mark_use(P, stream);
+      return mark_use(P, stream, !root_only);
     }
   }
   const bool stage = outside && d_br;
@@ -1767,7 +1794,7 @@ int run_post(subby_plan *P, const int32_t *d_aln, int C, int node, float *d_node
   int rc;
   if ((rc = plan_walk(P, k, !(outside && d_node), outside, chunk, per_sm, &w))) return rc;
   const size_t stage_floats = stage ? (size_t)(R - 1) * chunk * A : 0;
-  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + 256, stream)))
+  if ((rc = P->grow_work(w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + 256, stream)))
     return rc;
   char *base = place_walk(k, w, P->work.p);
   float *sa = stage ? (float *)base : nullptr;
@@ -1788,7 +1815,7 @@ int run_post(subby_plan *P, const int32_t *d_aln, int C, int node, float *d_node
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("posterior launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
   }
-  return mark_use(P, stream);
+  return mark_use(P, stream, true);
 }
 
 // Irreversible models, Counts / BranchCounts: the walk (mode 3) stages
@@ -1835,7 +1862,7 @@ int run_cx(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_c
   const size_t unit_blocks = units ? ((size_t)chunk + P->cxu.G - 1) / P->cxu.G : 0;
   const size_t proj_bytes = al256((size_t)(R - 1) * unit_blocks * 2 * P->cxu.UP * accx_stride(P->cxu.G) * sizeof(float));
   const size_t cbuf_bytes = (counts && bt64) ? (size_t)chunk * A * A * sizeof(float2) : 0;
-  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + al256(cbuf_bytes) + 2 * proj_bytes + 256,
+  if ((rc = P->grow_work(w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + al256(cbuf_bytes) + 2 * proj_bytes + 256,
                     stream)))
     return rc;
   char *base = place_walk(k, w, P->work.p);
@@ -1903,7 +1930,7 @@ int run_cx(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_c
       g_launches += 2;
     }
   }
-  return mark_use(P, stream);
+  return mark_use(P, stream, true);
 }
 
 // Gradient of reversible large-alphabet plans: the walk's eigen staging
@@ -1933,7 +1960,7 @@ int run_big_grad(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, cons
   // general products here
   if ((rc = plan_walk(P, k, proj_supported(A), R > 1, chunk, H == 2 ? 1 : 2, &w, false))) return rc;
   const size_t stage_bytes = R > 1 ? al256((size_t)(R - 1) * chunk * A * sizeof(float)) : 0;
-  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * stage_bytes + 256, stream))) return rc;
+  if ((rc = P->grow_work(w.vec_bytes + w.word_bytes + 2 * stage_bytes + 256, stream))) return rc;
   char *base = place_walk(k, w, P->work.p);
   float *sa = (float *)base;
   float *sb = (float *)(base + stage_bytes);
@@ -1953,7 +1980,7 @@ int run_big_grad(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, cons
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("gradient launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
   }
-  return mark_use(P, stream);
+  return mark_use(P, stream, true);
 }
 
 // Distance gradient of complex-system plans (irreversible or per-branch
@@ -1985,7 +2012,7 @@ int run_cx_grad(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, const
   int rc;
   if ((rc = plan_walk(P, k, true, R > 1, chunk, per_sm, &w))) return rc;
   const size_t stage_floats = R > 1 ? (size_t)(R - 1) * chunk * A : 0;
-  if ((rc = P->grow(P->work, w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + 256, stream)))
+  if ((rc = P->grow_work(w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + 256, stream)))
     return rc;
   char *base = place_walk(k, w, P->work.p);
   float *sa = R > 1 ? (float *)base : nullptr;
@@ -2004,7 +2031,7 @@ int run_cx_grad(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, const
     if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("gradient launch failed: ") + cudaGetErrorString((cudaError_t)lr));
     g_launches += 1;
   }
-  return mark_use(P, stream);
+  return mark_use(P, stream, true);
 }
 
 // Columns per chunk of the host-pointer pipeline: whole waves of the
@@ -2093,7 +2120,8 @@ int run_common(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float 
   const size_t vbytes = p4 ? p4n * 16 : (tree && !L.global_slots) ? 0 : nsl * L.nworkers * P->A * sizeof(float);
   const size_t wbytes = p4 ? p4n * 4 : (tree && !L.global_slots) ? 0 : nsl * L.nworkers * 2 * sizeof(int);
   const size_t vb_al = (vbytes + 255) & ~(size_t)255;
-  if ((rc = P->grow(P->work, vb_al + wbytes + 256, stream))) return rc;
+  const bool scratch = vbytes > 0;
+  if (scratch && (rc = P->grow_work(vb_al + wbytes + 256, stream))) return rc;
   k.scrV = (float *)P->work.p;
   k.scrW = (int *)((char *)P->work.p + vb_al);
   if (grid_out) *grid_out = L.grid;
@@ -2107,7 +2135,7 @@ int run_common(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float 
   if (lr != 0) return fail(SUBBY_ERR_CUDA, std::string("kernel launch failed: ") +
                                                cudaGetErrorString((cudaError_t)lr));
   g_launches += 1;
-  return mark_use(P, stream);
+  return mark_use(P, stream, scratch);
 }
 
 }  // namespace
@@ -2166,7 +2194,7 @@ int plan_packed_params(subby_plan *P, const int32_t *d_aln, int C, float *d_logL
 // The plan's tables were read by work enqueued on `stream` up to here.
 int plan_mark_used(subby_plan *P, cudaStream_t stream) {
   std::lock_guard<std::mutex> g(P->lock);
-  return mark_use(P, stream);
+  return mark_use(P, stream, false);
 }
 }  // namespace subby
 
@@ -2223,7 +2251,7 @@ int subby_plan_run(subby_plan *P, const int32_t *aln, int C, float *logL, float 
   const size_t b_rp = rootProb ? (size_t)A * C * 4 : 0;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t total = al(b_aln) + al(b_mask) + al(b_ll) + al(b_ct) + al(b_rp);
-  if ((rc = P->grow(P->io, total, stream))) return rc;
+  if ((rc = P->grow_io(total, stream))) return rc;
   char *base = (char *)P->io.p;
   int32_t *d_aln = (int32_t *)base;
   base += al(b_aln);
@@ -2336,7 +2364,7 @@ int subby_plan_branch_counts(subby_plan *P, const int32_t *aln, int C, float *br
   const size_t b_aln = (size_t)R * C * sizeof(int32_t);
   const size_t b_mask = (mask_mode == SUBBY_MASK_GIVEN) ? (size_t)R * C : 0;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  if ((rc = P->grow(P->io, al(b_aln) + al(b_mask) + al(b_out), stream))) return rc;
+  if ((rc = P->grow_io(al(b_aln) + al(b_mask) + al(b_out), stream))) return rc;
   char *base = (char *)P->io.p;
   int32_t *d_aln = (int32_t *)base;
   uint8_t *d_mask = b_mask ? (uint8_t *)(base + al(b_aln)) : nullptr;
@@ -2386,7 +2414,7 @@ int subby_plan_posteriors(subby_plan *P, const int32_t *aln, int C, int node, fl
   const size_t b_node = nodePost ? rows * A * C * sizeof(float) : 0;
   const size_t b_br = branchPost ? rows * A * A * C * sizeof(float) : 0;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  if ((rc = P->grow(P->io, al(b_aln) + al(b_node) + al(b_br), stream))) return rc;
+  if ((rc = P->grow_io(al(b_aln) + al(b_node) + al(b_br), stream))) return rc;
   char *base = (char *)P->io.p;
   int32_t *d_aln = (int32_t *)base;
   float *d_node = b_node ? (float *)(base + al(b_aln)) : nullptr;
@@ -2428,7 +2456,7 @@ int subby_plan_grad(subby_plan *P, const int32_t *aln, int C, const float *g, fl
   int rc = 0;
   if (!dev) {
     const size_t b_aln = (size_t)R * C * 4, b_g = g ? (size_t)C * 4 : 0, b_ll = logL ? (size_t)C * 4 : 0;
-    if ((rc = P->grow(P->io, al(b_aln) + al(b_g) + al(b_ll), stream))) return rc;
+    if ((rc = P->grow_io(al(b_aln) + al(b_g) + al(b_ll), stream))) return rc;
     char *base = (char *)P->io.p;
     int32_t *a = (int32_t *)base;
     base += al(b_aln);
