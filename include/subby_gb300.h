@@ -388,6 +388,13 @@ int subby_debug_set_kernel(int which);
  * counterpart. */
 int subby_debug_fail_waits(int polls);
 
+/* Test hook of the out-of-memory path: with bytes > 0, workspace allocations
+ * (subby_plan_run and its relatives) of more than `bytes` bytes fail as if
+ * the device had no memory left; a workspace that a plan already holds stays
+ * (subby_plan_trim).  0 (the default) turns it off.  No reference
+ * counterpart. */
+int subby_debug_alloc_limit(size_t bytes);
+
 /* Number of kernel launches the most recent subby_plan_run /
  * subby_plan_grad on this thread enqueued (for launch accounting). */
 int subby_last_launch_count(void);

@@ -23,7 +23,8 @@ EXPORTS = (
     "subby_plan_destroy", "subby_plan_device_bytes", "subby_plan_trim", "subby_plan_branch_counts",
     "subby_plan_posteriors", "subby_plan_status", "subby_plan_set_root_prior", "subby_plan_run", "subby_plan_grad",
     "subby_loglike", "subby_counts", "subby_rootprob", "subby_last_launch_count",
-    "subby_debug_set_kernel", "subby_debug_fail_waits", "subby_counts_noalloc", "subby_mixture_posterior",
+    "subby_debug_set_kernel", "subby_debug_fail_waits", "subby_debug_alloc_limit",
+    "subby_counts_noalloc", "subby_mixture_posterior",
     "subby_tokenize", "subby_gather_rows", "subby_server_create", "subby_server_submit", "subby_server_wait",
     "subby_server_release", "subby_server_set", "subby_server_clock", "subby_server_stats",
     "subby_server_destroy", "subby_debug_packed_queue_wait",
@@ -77,6 +78,8 @@ def _declare(lib):
     lib.subby_debug_set_kernel.argtypes = [ct.c_int]
     lib.subby_debug_fail_waits.restype = ct.c_int
     lib.subby_debug_fail_waits.argtypes = [ct.c_int]
+    lib.subby_debug_alloc_limit.restype = ct.c_int
+    lib.subby_debug_alloc_limit.argtypes = [ct.c_size_t]
     lib.subby_plan_create.restype = ct.c_int
     lib.subby_plan_create.argtypes = [_p, _p, _p, _p, _p, ct.c_int, ct.c_int, ct.POINTER(ct.c_void_p)]
     lib.subby_plan_create_rows.restype = ct.c_int

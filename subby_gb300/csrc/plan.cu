@@ -9,6 +9,7 @@
 #include <atomic>
 #include <cmath>
 #include <complex>
+#include <cstdint>
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
@@ -39,6 +40,9 @@ int g_kernel_sel = 0;
 // Test hook (subby_debug_fail_waits): > 0 makes every tensor-core walk give
 // up a prologue wait after that many polls.
 std::atomic<int> g_dbg_wait_polls{0};
+// Test hook (subby_debug_alloc_limit): > 0 makes workspace allocations of
+// more bytes fail.
+std::atomic<size_t> g_dbg_alloc_limit{0};
 
 int fail(int code, const std::string &msg) {
   g_static_error = nullptr;
@@ -210,17 +214,22 @@ struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
   // Grow to `need` bytes in stream order on `s`, which comes after every
-  // enqueued use of the old block.
-  int grow(size_t need, cudaStream_t s, cudaMemPool_t pool) {
+  // enqueued use of the old block.  A quarter is added for later growth, up
+  // to `most` bytes where no call needs more than that.
+  int grow(size_t need, cudaStream_t s, cudaMemPool_t pool, size_t most = SIZE_MAX) {
     if (need <= bytes) return 0;
     if (p) cudaFreeAsync(p, s);
     p = nullptr;
     bytes = 0;
-    size_t want = need + need / 4;
-    cudaError_t e = pool_alloc(&p, want, pool, s);
+    size_t want = std::max(need, std::min(need + need / 4, most));
+    const size_t limit = g_dbg_alloc_limit.load();
+    auto alloc = [&](size_t n) {
+      return limit > 0 && n > limit ? cudaErrorMemoryAllocation : pool_alloc(&p, n, pool, s);
+    };
+    cudaError_t e = alloc(want);
     if (e != cudaSuccess) {
       cudaGetLastError();
-      e = pool_alloc(&p, need, pool, s);
+      e = alloc(need);
       if (e != cudaSuccess) {
         cudaGetLastError();
         p = nullptr;
@@ -319,11 +328,11 @@ struct subby_plan {
     return e;
   }
   // `s` after the latest use of `work`, which then holds `need` bytes
-  int grow_work(size_t need, cudaStream_t s) {
+  int grow_work(size_t need, cudaStream_t s, size_t most = SIZE_MAX) {
     unsigned long long id = 0;
     cudaError_t e = cudaStreamGetId(s, &id);
     if (e == cudaSuccess && work_use.set && work_use.stream != id) e = cudaStreamWaitEvent(s, work_use.e, 0);
-    return e == cudaSuccess ? work.grow(need, s, pool) : cuda_fail(e, "workspace order");
+    return e == cudaSuccess ? work.grow(need, s, pool, most) : cuda_fail(e, "workspace order");
   }
   int grow_io(size_t need, cudaStream_t s) {
     if (need > io.bytes) wait_runs(s);
@@ -388,6 +397,11 @@ int subby_debug_set_kernel(int which) {
   return SUBBY_OK;
 }
 int subby_last_launch_count(void) { return g_launches; }
+
+int subby_debug_alloc_limit(size_t bytes) {
+  g_dbg_alloc_limit.store(bytes);
+  return SUBBY_OK;
+}
 
 int subby_debug_fail_waits(int polls) {
   if (polls < 0 || polls > 4096) return fail(SUBBY_ERR_ARG, "polls must be 0..4096");
@@ -1551,6 +1565,28 @@ int plan_pass4(subby_plan *P, int mode, bool post, int C, Launch &L) {
   return 0;
 }
 
+size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+// The node slots of a k_pass4 run on `stream`.  Out of device memory the grid
+// is halved, to no fewer than `least` CTAs (a column's results do not depend
+// on the grid).
+int place_pass4(subby_plan *P, Launch &L, int least, cudaStream_t stream) {
+  auto slots = [&](int grid) { return (size_t)L.kp.nsteps * L.columns * L.block * grid; };
+  auto bytes = [&](int grid) { return al256(slots(grid) * 16) + slots(grid) * 4 + 256; };
+  // (no run of the plan has more threads on an SM than 384 of two columns)
+  const size_t most = (size_t)L.kp.nsteps * 2 * 384 * P->nsm * 20 + 512;
+  int rc;
+  while ((rc = P->grow_work(bytes(L.grid), stream, most)) == SUBBY_ERR_NOMEM && L.grid > least)
+    L.grid = std::max(L.grid / 2, least);
+  if (rc) return rc;
+  clear_error();
+  L.nworkers = L.grid * L.block;
+  L.kp.nworkers = L.nworkers;
+  L.kp.scrV = (float *)P->work.p;
+  L.kp.scrW = (int *)((char *)P->work.p + al256(slots(L.grid) * 16));
+  return 0;
+}
+
 // Large alphabets (A = 16, 20, 32, 64): k_walk (tree walk, 128 columns per
 // CTA, stored-node slots in global memory) then, for Counts, k_acc over the
 // staged per-branch vectors.  Columns are processed in chunks so that the
@@ -1618,7 +1654,6 @@ struct WalkPlan {
   int grid = 1;
   size_t vec_bytes = 0, word_bytes = 0;
 };
-size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 int plan_walk(const subby_plan *P, KParams &k, bool q, bool outside, int chunk, int per_sm, WalkPlan *w,
               bool closed_form = true) {
@@ -1758,11 +1793,8 @@ int run_post(subby_plan *P, const int32_t *d_aln, int C, int node, float *d_node
       if (root_only) {
         lr = launch_inside4(k, L4.columns, L4.grid, L4.block, L4.smem, stream);
       } else {
-        const size_t n4 = (size_t)k.nsteps * L4.columns * L4.nworkers;
         int rc;
-        if ((rc = P->grow_work(al256(n4 * 16) + n4 * 4 + 256, stream))) return rc;
-        k.scrV = (float *)P->work.p;
-        k.scrW = (int *)((char *)P->work.p + al256(n4 * 16));
+        if ((rc = place_pass4(P, L4, 1, stream))) return rc;
         lr = launch_pass4(k, P->prog_i.data(), P->prog_other.data(), P->hVd.data(), P->hVu.data(), P->hpi, false, kMaskNone, true, L4.columns, L4.grid,
                           L4.block, L4.smem, stream);
       }
@@ -2083,8 +2115,22 @@ int run_common(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float 
   if (tree && plan_inside4(P, mode, C, L) == 0) {
     inside4 = true;
   } else if (tree && plan_pass4(P, mode, false, C, L = Launch()) == 0) {
-    p4 = true;
-  } else if (tree && (rc = plan_tree4(P, mode, C, L = Launch())) == 0) {
+    // without the memory for one CTA per SM: k_tree4, which needs none, where
+    // the tree fits it
+    rc = place_pass4(P, L, P->nsm, stream);
+    if (rc == SUBBY_ERR_NOMEM) {
+      Launch T;
+      if (plan_tree4(P, mode, C, T) == 0) {
+        L = T;
+        tree4 = true;
+        clear_error();
+      } else {
+        rc = place_pass4(P, L, 1, stream);
+      }
+    }
+    if (rc && !tree4) return rc;
+    p4 = !tree4;
+  } else if (tree && plan_tree4(P, mode, C, L = Launch()) == 0) {
     tree4 = true;
   } else {
     L = Launch();
@@ -2116,14 +2162,13 @@ int run_common(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float 
   k.grad_C = d_gC;
   // scratch
   const size_t nsl = (size_t)std::max(tree ? P->prog_slots : P->nslots, 1);
-  const size_t p4n = p4 ? (size_t)k.nsteps * L.columns * L.nworkers : 0;
-  const size_t vbytes = p4 ? p4n * 16 : (tree && !L.global_slots) ? 0 : nsl * L.nworkers * P->A * sizeof(float);
-  const size_t wbytes = p4 ? p4n * 4 : (tree && !L.global_slots) ? 0 : nsl * L.nworkers * 2 * sizeof(int);
-  const size_t vb_al = (vbytes + 255) & ~(size_t)255;
-  const bool scratch = vbytes > 0;
-  if (scratch && (rc = P->grow_work(vb_al + wbytes + 256, stream))) return rc;
-  k.scrV = (float *)P->work.p;
-  k.scrW = (int *)((char *)P->work.p + vb_al);
+  const bool scratch = p4 || !tree || L.global_slots;
+  if (scratch && !p4) {
+    const size_t vbytes = nsl * L.nworkers * P->A * sizeof(float), wbytes = nsl * L.nworkers * 2 * sizeof(int);
+    if ((rc = P->grow_work(al256(vbytes) + wbytes + 256, stream))) return rc;
+    k.scrV = (float *)P->work.p;
+    k.scrW = (int *)((char *)P->work.p + al256(vbytes));
+  }
   if (grid_out) *grid_out = L.grid;
   int lr = p4 ? launch_pass4(k, P->prog_i.data(), P->prog_other.data(), P->hVd.data(), P->hVu.data(), P->hpi, (mode & kModeF81) != 0, mask_mode, false,
                              L.columns, L.grid, L.block, L.smem, stream)
