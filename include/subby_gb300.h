@@ -379,11 +379,12 @@ int subby_debug_packed_queue_wait(int polls, int grid, int *gave_up);
 int subby_debug_set_kernel(int which);
 
 /* Test hook of the bounded-wait failure path: with polls > 0, every
- * tensor-core tree walk (A = 64) launched afterwards first waits on an
- * mbarrier that nothing arms, while no copy or MMA is in flight, gives up
- * after `polls` polls, frees its tensor memory and skips its work, so that
- * subby_plan_status (device pointers) or the call itself (host pointers)
- * reports SUBBY_ERR_TIMEOUT and the outputs are left unwritten.  0 (the
+ * tensor-core tree walk (A = 64) and every four-lane walk with a matrix ring
+ * (A = 16, 20, 32) launched afterwards first waits on an mbarrier that
+ * nothing arms, while no copy or MMA is in flight, gives up after `polls`
+ * polls, frees its tensor memory and skips its work, so that
+ * subby_plan_status (device pointers) or the call itself (host pointers, and
+ * every gradient) reports SUBBY_ERR_TIMEOUT and the outputs are invalid.  0 (the
  * default) turns it off; polls must be 0..4096.  No reference
  * counterpart. */
 int subby_debug_fail_waits(int polls);

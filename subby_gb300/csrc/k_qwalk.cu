@@ -144,7 +144,7 @@ __global__ void __launch_bounds__((q_threads<CPL, F81M>()), MINB)
   using V = QV<A, CPL>;
   extern __shared__ __align__(128) float sm[];
   __shared__ __align__(8) uint64_t s_full[kQS], s_empty[kQS];
-  __shared__ int s_err;
+  __shared__ int s_err, s_skip;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sg = lane >> 3, cg = lane & 7;
   const float *MT = P.tab + P.off.MT;
@@ -168,9 +168,18 @@ __global__ void __launch_bounds__((q_threads<CPL, F81M>()), MINB)
                    "r"(kQW));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    // Test hook of the failure path: a wait for the first step's matrices,
+    // which nothing has requested yet (no copy is in flight), for a few polls;
+    // it gives up and the CTA skips its work.
+    s_skip = !F81M && P.dbg_wait_polls > 0 &&
+             !mbar_wait((uint32_t)__cvta_generic_to_shared(&s_full[0]), 0, P.dbg_wait_polls);
   }
   __syncwarp();
   __syncthreads();
+  if (!F81M && s_skip) {
+    if (threadIdx.x == 0 && P.err) atomicAdd(P.err, 1);
+    return;
+  }
 
   // Ring of the steps' matrices in the order of their use (every tile: the
   // steps forwards, then backwards).  One thread refills it: with one column

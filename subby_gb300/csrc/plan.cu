@@ -37,8 +37,8 @@ thread_local int g_launches = 0;
 // cores) for large A, 3 tree program with global-memory slots, 4 generic
 // tree program with tensor-memory slots (bypassing the A = 4 specialisation).
 int g_kernel_sel = 0;
-// Test hook (subby_debug_fail_waits): > 0 makes every tensor-core walk give
-// up a prologue wait after that many polls.
+// Test hook (subby_debug_fail_waits): > 0 makes every walk whose matrices
+// come by bulk copies give up a prologue wait after that many polls.
 std::atomic<int> g_dbg_wait_polls{0};
 // Test hook (subby_debug_alloc_limit): > 0 makes workspace allocations of
 // more bytes fail.
@@ -2088,6 +2088,23 @@ int ensure_pipeline(subby_plan *P, int nev) {
   return 0;
 }
 
+// A status word read back: clears the device's (in stream order on `stream`)
+// and reports a bounded wait that gave up.
+int report_waits(subby_plan *P, int gave_up, cudaStream_t stream) {
+  if (!gave_up) return SUBBY_OK;
+  cudaMemsetAsync(P->d_err, 0, sizeof(int), stream);
+  cudaStreamSynchronize(stream);
+  return fail(SUBBY_ERR_TIMEOUT, "a bounded device wait gave up in " + std::to_string(gave_up) + " CTA(s)");
+}
+
+// Waits for the work on `stream` and checks its bounded waits.
+int finish_host_call(subby_plan *P, cudaStream_t stream) {
+  int gave_up = 0;
+  CU(cudaMemcpyAsync(&gave_up, P->d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  CU(cudaStreamSynchronize(stream));
+  return report_waits(P, gave_up, stream);
+}
+
 int run_common(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_counts,
                float *d_root, int mode, int mask_mode, const uint8_t *d_mask, const float *d_g,
                double *d_gt, double *d_gC, int *grid_out, cudaStream_t stream) {
@@ -2357,19 +2374,9 @@ int subby_plan_run(subby_plan *P, const int32_t *aln, int C, float *logL, float 
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) return finish(cuda_fail(e, "chunk pipeline"));
   }
-  if (P->d_err) {
-    int dev_err = 0;
-    CU(cudaMemcpyAsync(&dev_err, P->d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    CU(cudaStreamSynchronize(stream));
-    if (dev_err) {
-      cudaMemsetAsync(P->d_err, 0, sizeof(int), stream);
-      cudaStreamSynchronize(stream);
-      if (dev != P->device) cudaSetDevice(dev);
-      return fail(SUBBY_ERR_TIMEOUT, "a bounded device wait gave up (tensor-core walk)");
-    }
-  }
+  rc = finish_host_call(P, stream);
   if (dev != P->device) cudaSetDevice(dev);
-  return SUBBY_OK;
+  return rc;
 }
 
 int subby_plan_branch_counts(subby_plan *P, const int32_t *aln, int C, float *branchCounts, int counts_kind,
@@ -2423,9 +2430,9 @@ int subby_plan_branch_counts(subby_plan *P, const int32_t *aln, int C, float *br
     return rc;
   }
   CU(cudaMemcpyAsync(branchCounts, d_out, b_out, cudaMemcpyDeviceToHost, stream));
-  CU(cudaStreamSynchronize(stream));
+  rc = finish_host_call(P, stream);
   if (dev != P->device) cudaSetDevice(dev);
-  return SUBBY_OK;
+  return rc;
 }
 
 int subby_plan_posteriors(subby_plan *P, const int32_t *aln, int C, int node, float *nodePost, float *branchPost,
@@ -2471,9 +2478,9 @@ int subby_plan_posteriors(subby_plan *P, const int32_t *aln, int C, int node, fl
   }
   if (b_node) CU(cudaMemcpyAsync(nodePost, d_node, b_node, cudaMemcpyDeviceToHost, stream));
   if (b_br) CU(cudaMemcpyAsync(branchPost, d_br, b_br, cudaMemcpyDeviceToHost, stream));
-  CU(cudaStreamSynchronize(stream));
+  rc = finish_host_call(P, stream);
   if (dev != P->device) cudaSetDevice(dev);
-  return SUBBY_OK;
+  return rc;
 }
 
 int subby_plan_grad(subby_plan *P, const int32_t *aln, int C, const float *g, float *logL,
@@ -2517,27 +2524,35 @@ int subby_plan_grad(subby_plan *P, const int32_t *aln, int C, const float *g, fl
   if (P->irrev) {
     // complex-system plans: distance gradient only (dldS: the gradient with
     // respect to exchangeabilities does not apply; zeros)
+    // (behind the gradient: the status word of its kernels)
     double *d_gt = nullptr;
-    CU(pool_alloc((void **)&d_gt, sizeof(double) * R, P->pool, stream));
+    CU(pool_alloc((void **)&d_gt, sizeof(double) * (R + 1), P->pool, stream));
     CU(cudaMemsetAsync(d_gt, 0, sizeof(double) * R, stream));
     rc = run_cx_grad(P, d_aln, C, logL ? d_ll : nullptr, d_g, d_gt, stream);
+    std::vector<double> res((size_t)R + 1);
     cudaError_t e = cudaSuccess;
-    if (rc == 0) e = cudaMemcpyAsync(dldt, d_gt, sizeof(double) * R, cudaMemcpyDeviceToHost, stream);
+    if (rc == 0) e = cudaMemcpyAsync(d_gt + R, P->d_err, sizeof(int), cudaMemcpyDeviceToDevice, stream);
+    if (rc == 0 && e == cudaSuccess)
+      e = cudaMemcpyAsync(res.data(), d_gt, sizeof(double) * (R + 1), cudaMemcpyDeviceToHost, stream);
     if (rc == 0 && e == cudaSuccess && logL && !dev)
       e = cudaMemcpyAsync(logL, d_ll, (size_t)C * 4, cudaMemcpyDeviceToHost, stream);
     cudaFreeAsync(d_gt, stream);
     cudaError_t e2 = cudaStreamSynchronize(stream);
     if (rc) return rc;
     if (e != cudaSuccess || e2 != cudaSuccess) return cuda_fail(e != cudaSuccess ? e : e2, "gradient readback");
+    int gave_up = 0;
+    std::memcpy(&gave_up, &res[R], sizeof(int));
+    if ((rc = report_waits(P, gave_up, stream))) return rc;
+    std::copy(res.begin(), res.begin() + R, dldt);
     dldt[0] = 0.0;
     for (int i = 0; i < A * A; ++i) dldS[i] = 0.0;
     return SUBBY_OK;
   }
   if (big_supported(A) && g_kernel_sel == 0) {
     // walk + per-branch sums and their contraction (k_grad.cu), FP64; d_X is
-    // followed by grad_t (R) and Cg (A x A)
+    // followed by grad_t (R), Cg (A x A) and the status word of the kernels
     double *d_X = nullptr;
-    const size_t nx = (size_t)R * A * A, nout = (size_t)R + (size_t)A * A;
+    const size_t nx = (size_t)R * A * A, nout = (size_t)R + (size_t)A * A + 1;
     CU(pool_alloc((void **)&d_X, sizeof(double) * (nx + nout), P->pool, stream));
     CU(cudaMemsetAsync(d_X, 0, sizeof(double) * (nx + nout), stream));
     rc = run_big_grad(P, d_aln, C, logL ? d_ll : nullptr, d_g, d_X, stream);
@@ -2548,13 +2563,18 @@ int subby_plan_grad(subby_plan *P, const int32_t *aln, int C, const float *g, fl
     }
     std::vector<double> res(nout, 0.0);
     cudaError_t e = cudaSuccess;
-    if (rc == 0) e = cudaMemcpyAsync(res.data(), d_X + nx, sizeof(double) * nout, cudaMemcpyDeviceToHost, stream);
+    if (rc == 0) e = cudaMemcpyAsync(d_X + nx + nout - 1, P->d_err, sizeof(int), cudaMemcpyDeviceToDevice, stream);
+    if (rc == 0 && e == cudaSuccess)
+      e = cudaMemcpyAsync(res.data(), d_X + nx, sizeof(double) * nout, cudaMemcpyDeviceToHost, stream);
     if (rc == 0 && e == cudaSuccess && logL && !dev)
       e = cudaMemcpyAsync(logL, d_ll, (size_t)C * 4, cudaMemcpyDeviceToHost, stream);
     cudaFreeAsync(d_X, stream);
     cudaError_t e2 = cudaStreamSynchronize(stream);
     if (rc) return rc;
     if (e != cudaSuccess || e2 != cudaSuccess) return cuda_fail(e != cudaSuccess ? e : e2, "gradient readback");
+    int gave_up = 0;
+    std::memcpy(&gave_up, &res[nout - 1], sizeof(int));
+    if ((rc = report_waits(P, gave_up, stream))) return rc;
     std::copy(res.begin(), res.begin() + R, dldt);
     dldt[0] = 0.0;
     const double *Cg = res.data() + R;
