@@ -1512,6 +1512,17 @@ int plan_inside4(subby_plan *P, int mode, int C, Launch &L) {
   while (bytes() > (size_t)maxsm && L.block > 64) L.block /= 2;
   L.smem = bytes();
   if (L.smem > (size_t)maxsm) return 1;
+  if (2 * (L.smem + 1024) > (size_t)maxsm + 1024) {
+    // Large tables, one CTA per SM: waves of equal size, as a few CTAs more
+    // than there are SMs cost a whole wave (R = 1599, 20000 columns: CTAs of
+    // 128 587 us, of 160 320 us).
+    L.block = 256;
+    while (bytes() > (size_t)maxsm) L.block -= 32;
+    const long long wave = (long long)P->nsm * L.block * per, waves = (C + wave - 1) / wave;
+    const long long cols = waves * P->nsm * per;
+    L.block = std::min(L.block, std::max(32, (int)((C + cols - 1) / cols + 31) / 32 * 32));
+    L.smem = bytes();
+  }
   const int per_sm = std::max(1, std::min((per == 2 ? 768 : 1024) / L.block, (int)(((size_t)maxsm + 1024) / (L.smem + 1024))));
   L.kernel = 4;
   L.small = false;
