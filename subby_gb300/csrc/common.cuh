@@ -260,10 +260,11 @@ int launch_accx(const KParams &p, int A, const CxUnits &cu, const CxHost &h, con
                 float *pa, float *pb, int c_base, int c_count, int nsm, cudaStream_t s);
 // reversible large-alphabet gradient (k_grad.cu): X_n += sum_c g_c D~_nc (x) U~_nc
 // from the eigen staging, X (R x A x A) FP64; then the contraction of every
-// X_n into grad_t (R) and Cg (A x A)
+// X_n (overwritten) into grad_t (R) and Cg (A x A, then the status word *err)
 int launch_xgram(const KParams &p, int A, const float *sa, const float *sb, const float *g, int c_base, int c_count,
                  double *X, int nsm, cudaStream_t s);
-int launch_xform(const double *X, const double *tab64, int R, int A, double *grad_t, double *Cg, cudaStream_t s);
+int launch_xform(double *X, const double *tab64, int R, int A, double *grad_t, double *Cg, const int *err,
+                 cudaStream_t s);
 // distance gradient from the raw staging: grad_t[n] += sum_c g_c (D s)^T G_n U
 int launch_grad_cx(const KParams &p, int A, const float *sa, const float *sb, const float *gq, const float *g,
                    int c_base, int c_count, double *grad_t, int grid, cudaStream_t s);

@@ -4,7 +4,8 @@
 // functions of one A x A matrix per branch,
 //   X_n = sum_c g_c D~_nc (x) U~_nc :
 //   d/dt_n = sum_k mu_k e^{mu_k t_n} X_n[k][k],  d/dS~ = V (sum_n J_n o X_n) V^T
-// (k_xform contracts X_n with the branch's coefficients, in FP64).
+// (k_xform contracts X_n with the branch's coefficients, k_xsum adds the
+// branches up, in FP64).
 // k_xgram: per (branch, block of 4096 columns) each thread owns a 4 x 4 block
 // of (k, l) for a subset of the columns (two 16-byte loads and 16 FMAs per
 // column), the column subsets are reduced in shared memory and the block's
@@ -90,8 +91,8 @@ __global__ void __launch_bounds__(kXThreads) k_xgram(const float *__restrict__ s
 // load pipe at 1.7 TB/s.  Here a lane owns a 4 x LW block (LW = A, at A = 32
 // half a row): 4 + LW floats for 4 LW multiply-adds, and a CTA takes NB
 // branches of the same columns, whose rows come through a ring of bulk
-// copies.  Measured per 50000 columns at A = 20, R = 399 (3.2 GB): see
-// launch_xgram.
+// copies.  The subsets are added in their order, as k_xgram does, so that the
+// gradients of up to 4096 columns are the same in every call.
 template <int A>
 struct XG {
   static constexpr int LW = A == 32 ? 16 : A;
@@ -105,6 +106,8 @@ struct XG {
   static constexpr int ROWS = TC * A;                           // floats of a stage's rows of one vector and branch
   static constexpr int STAGE = NB * 2 * ROWS;
   static constexpr int FLOATS = NS * STAGE;
+  static constexpr int OUT = NT * LW;                           // a branch's entries of one of the four rows of every block
+  static_assert(NB * GROUPS * OUT <= STAGE, "the subsets' sums take a ring stage");
 };
 
 template <int A>
@@ -202,25 +205,40 @@ __global__ void __launch_bounds__(kXThreads, 2)
           }
         }
     }
-    // (FP64, as k_xgram sums its subsets; the order of FP64 additions is free)
-    if (busy) {
-      double *o = X + ((size_t)(n + 1) * A + 4 * kt) * A + lt * LW;
+    // The subsets' sums through the ring stage just read, which the next
+    // item's first barrier hands to the bulk copies: one row of the 4 x LW
+    // blocks at a time, [branch][subset][block][LW].
+    float *part = sm + ((pos + G::NS - 1) % G::NS) * G::STAGE;
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < 4; ++q) {
+      __syncthreads();
+      if (busy)
 #pragma unroll
-        for (int j = 0; j < LW; ++j)
-          atomicAdd(o + q * A + j, (double)((j & 1) ? acc[q][j >> 1].y : acc[q][j >> 1].x));
+        for (int j = 0; j < LW / 4; ++j)
+          *reinterpret_cast<float4 *>(part + ((br * G::GROUPS + grp) * G::NT + tile) * LW + 4 * j) =
+              make_float4(acc[q][2 * j].x, acc[q][2 * j].y, acc[q][2 * j + 1].x, acc[q][2 * j + 1].y);
+      __syncthreads();
+      for (int e = t; e < G::NB * G::OUT; e += kXThreads) {
+        const int b = e / G::OUT, r2 = e % G::OUT, b2 = it / nblk * G::NB + b;
+        if (b2 >= R - 1) break;
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < G::GROUPS; ++i) s += (double)part[(b * G::GROUPS + i) * G::OUT + r2];
+        const int tl = r2 / LW;   // its block
+        atomicAdd(X + ((size_t)(b2 + 1) * A + 4 * (tl / (A / LW)) + q) * A + (tl % (A / LW)) * LW + r2 % LW, s);
+      }
     }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
   if (t == 0 && s_err && err) atomicAdd(err, 1);
 }
 
-// One CTA per branch, FP64: grad_t[n] = sum_k mu_k e^{mu_k t_n} X_n[k][k] and
-// Cg += J_n o X_n with the 1e-8 degeneracy rule of J
+// One CTA per branch, FP64: grad_t[n] = sum_k mu_k e^{mu_k t_n} X_n[k][k], and
+// X_n becomes J_n o X_n with the 1e-8 degeneracy rule of J
 // (subby/oracle/oracle.py:931-959).  tab64: V, S, mu, t, pi.
-__global__ void k_xform(const double *__restrict__ X, const double *__restrict__ tab64, int R, int A,
-                        double *__restrict__ grad_t, double *__restrict__ Cg) {
+__global__ void k_xform(double *__restrict__ X, const double *__restrict__ tab64, int R, int A,
+                        double *__restrict__ grad_t) {
   extern __shared__ double sd[];
   double *x = sd, *ek = sd + A * A;   // X_n, e^{mu t_n}
   const double *mu = tab64 + 2 * A * A, *tt = mu + A;
@@ -233,13 +251,34 @@ __global__ void k_xform(const double *__restrict__ X, const double *__restrict__
     const int k = e / A, l = e % A;
     const double d = mu[k] - mu[l];
     const double J = fabs(d) < 1e-8 ? t * ek[k] : (ek[k] - ek[l]) / d;
-    atomicAdd(Cg + e, J * x[e]);
+    X[(size_t)n * A * A + e] = J * x[e];
   }
   if (threadIdx.x == 0) {
     double s = 0.0;
     for (int k = 0; k < A; ++k) s += mu[k] * ek[k] * x[k * A + k];
     grad_t[n] = s;
   }
+}
+
+// Cg = sum_n of k_xform's matrices, in a fixed order: a lane per entry, each
+// warp every kSumWarps-th branch, then the warps in turn.  Behind Cg goes the
+// status word of the kernels before, for the host's one readback.
+constexpr int kSumWarps = 8;
+__global__ void __launch_bounds__(32 * kSumWarps) k_xsum(const double *__restrict__ X, int R, int AA,
+                                                         double *__restrict__ Cg, const int *__restrict__ err) {
+  __shared__ double part[kSumWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+  double s = 0.0;
+  if (e < AA)
+#pragma unroll 8
+    for (int n = 1 + w; n < R; n += kSumWarps) s += X[(size_t)n * AA + e];
+  part[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && e < AA) {
+    for (int i = 1; i < kSumWarps; ++i) s += part[i][lane];
+    Cg[e] = s;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<int *>(Cg + AA) = *err;
 }
 
 template <int A>
@@ -257,11 +296,15 @@ int xgram_wide(const KParams &p, const float *sa, const float *sb, const float *
 
 }  // namespace
 
-int launch_xform(const double *X, const double *tab64, int R, int A, double *grad_t, double *Cg, cudaStream_t s) {
+int launch_xform(double *X, const double *tab64, int R, int A, double *grad_t, double *Cg, const int *err,
+                 cudaStream_t s) {
   const size_t smem = (size_t)(A * A + A) * sizeof(double);
   cudaError_t e = cudaFuncSetAttribute(k_xform, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  k_xform<<<R - 1, 256, smem, s>>>(X, tab64, R, A, grad_t, Cg);
+  k_xform<<<R - 1, 256, smem, s>>>(X, tab64, R, A, grad_t);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return (int)e;
+  k_xsum<<<(A * A + 31) / 32, 32 * kSumWarps, 0, s>>>(X, R, A * A, Cg, err);
   return (int)cudaGetLastError();
 }
 

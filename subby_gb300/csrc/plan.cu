@@ -2568,14 +2568,13 @@ int subby_plan_grad(subby_plan *P, const int32_t *aln, int C, const float *g, fl
     CU(cudaMemsetAsync(d_X, 0, sizeof(double) * (nx + nout), stream));
     rc = run_big_grad(P, d_aln, C, logL ? d_ll : nullptr, d_g, d_X, stream);
     if (rc == 0 && R > 1) {
-      const int lr = launch_xform(d_X, P->d_tab64, R, A, d_X + nx, d_X + nx + R, stream);
+      const int lr = launch_xform(d_X, P->d_tab64, R, A, d_X + nx, d_X + nx + R, P->d_err, stream);
       if (lr != 0) rc = fail(SUBBY_ERR_CUDA, std::string("gradient launch failed: ") + cudaGetErrorString((cudaError_t)lr));
-      else g_launches += 1;
+      else g_launches += 2;
     }
     std::vector<double> res(nout, 0.0);
     cudaError_t e = cudaSuccess;
-    if (rc == 0) e = cudaMemcpyAsync(d_X + nx + nout - 1, P->d_err, sizeof(int), cudaMemcpyDeviceToDevice, stream);
-    if (rc == 0 && e == cudaSuccess)
+    if (rc == 0)
       e = cudaMemcpyAsync(res.data(), d_X + nx, sizeof(double) * nout, cudaMemcpyDeviceToHost, stream);
     if (rc == 0 && e == cudaSuccess && logL && !dev)
       e = cudaMemcpyAsync(logL, d_ll, (size_t)C * 4, cudaMemcpyDeviceToHost, stream);
