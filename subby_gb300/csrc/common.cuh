@@ -237,8 +237,8 @@ int launch_bt_cx(const KParams &p, int A, const float2 *cbuf, int c_base, int c_
                  cudaStream_t s);
 // irreversible counts at A = 16, 20, 32 for eigensystems in conjugate pairs
 // (k_accx.cu): the units' tables on the device (U units, padded to an even
-// UP, the first `pairs` of them conjugate pairs, then reals; G columns per
-// block) and the real-form projection matrices on the host
+// UP, the first `pairs` of them conjugate pairs, then reals; up to G columns
+// per block) and the real-form projection matrices on the host
 struct CxUnits {
   int U, UP, pairs, G;
   const float *J;        // R x UP x UP x (J_kl, J_kl')
@@ -256,6 +256,7 @@ bool accx_supported(int A);
 // four apart start 8 banks apart
 __host__ __device__ constexpr int accx_stride(int G) { return G + 2; }
 int accx_group(int A, int UP);
+int accx_columns(int G, int C, int nsm);   // of a block, for a call of C columns
 int launch_accx(const KParams &p, int A, const CxUnits &cu, const CxHost &h, const float *sa, const float *sb,
                 float *pa, float *pb, int c_base, int c_count, int nsm, cudaStream_t s);
 // reversible large-alphabet gradient (k_grad.cu): X_n += sum_c g_c D~_nc (x) U~_nc

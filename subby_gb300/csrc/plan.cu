@@ -1902,8 +1902,10 @@ int run_cx(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_c
   int rc;
   if ((rc = plan_walk(P, k, true, counts, chunk, per_sm, &w))) return rc;
   const size_t stage_floats = counts ? (size_t)(R - 1) * chunk * A : 0;
-  const size_t unit_blocks = units ? ((size_t)chunk + P->cxu.G - 1) / P->cxu.G : 0;
-  const size_t proj_bytes = al256((size_t)(R - 1) * unit_blocks * 2 * P->cxu.UP * accx_stride(P->cxu.G) * sizeof(float));
+  CxUnits cu = P->cxu;
+  if (units) cu.G = accx_columns(cu.G, chunk, P->nsm);
+  const size_t unit_blocks = units ? ((size_t)chunk + cu.G - 1) / cu.G : 0;
+  const size_t proj_bytes = al256((size_t)(R - 1) * unit_blocks * 2 * cu.UP * accx_stride(cu.G) * sizeof(float));
   const size_t cbuf_bytes = (counts && bt64) ? (size_t)chunk * A * A * sizeof(float2) : 0;
   if ((rc = P->grow_work(w.vec_bytes + w.word_bytes + 2 * al256(stage_floats * 4) + al256(cbuf_bytes) + 2 * proj_bytes + 256,
                     stream)))
@@ -1914,7 +1916,6 @@ int run_cx(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_c
   float *sb = counts ? (float *)base : nullptr;
   base += al256(stage_floats * 4);
   float2 *cbuf = cbuf_bytes ? (float2 *)base : nullptr;
-  CxUnits cu = P->cxu;
   const int xi = k.cx_exact ? 1 : 0;
   if (units) {
     const int UP = cu.UP;
