@@ -985,7 +985,8 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
         }
     }
     std::vector<int> rep_u, partner;
-    if (!ir->per_row && accx_supported(A) && R > 1 && cx_cond(*ir, A) <= kCxCond && cx_pair_up(*ir, A, rep_u, partner)) {
+    if (!ir->per_row && accx_supported(A) && R > 1 && cx_cond(*ir, A) <= kCxCond && cx_pair_up(*ir, A, rep_u, partner) &&
+        accx_group(A, ((int)rep_u.size() + 1) & ~1) > 0) {
       CxUnits &cu = P->cxu;
       cu.U = (int)rep_u.size();
       cu.UP = (cu.U + 1) & ~1;
@@ -1882,15 +1883,18 @@ int run_cx(subby_plan *P, const int32_t *d_aln, int C, float *d_logL, float *d_c
   k.npost = nullptr;
   k.npost_node = -1;
   // conjugate-paired systems at A = 16, 20, 32: k_accx
-  const bool units = counts && !pb && P->d_cxu && P->cxu.G > 0;
+  const bool units = counts && !pb && P->d_cxu;
   const bool bt64 = cx_bt64(A) && !P->rows;   // per-branch reversible systems are well conditioned
   const bool tc = (A == 64) && P->d_tab16 && (g_kernel_sel == 0 || g_kernel_sel == 5);
   const int tile = big_tile();
   const int H = (A + 31) / 32;
   int chunk = C;
   if (counts) {
-    // (with the projected vectors beside the raw ones for k_accx)
-    const size_t per_col = (size_t)2 * (R - 1) * (A + (units ? 2 * P->cxu.UP : 0)) * sizeof(float);
+    // (with the projected vectors and the padding of the smallest blocks
+    // beside the raw ones for k_accx)
+    const int g = std::min(P->cxu.G, 16);
+    const size_t proj = units ? (size_t)(2 * P->cxu.UP * accx_stride(g) + g - 1) / g : 0;
+    const size_t per_col = (size_t)2 * (R - 1) * (A + proj) * sizeof(float);
     size_t cmax = std::max<size_t>(tile, kStageBudget / per_col);
     cmax = cmax / tile * tile;
     const size_t nch = ((size_t)C + cmax - 1) / cmax;

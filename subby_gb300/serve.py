@@ -43,7 +43,7 @@ import numpy as np
 
 from . import _lib
 from .api import Plan
-from .models import ensure_diag
+from .models import ensure_diag, is_irrev
 from . import batch
 
 
@@ -131,15 +131,19 @@ def job_cost_ms(R: int, C: int, A: int, f81: bool = False) -> float:
     return _NS_PER_COL_NODE[key] * R * C * 1e-6 + 4.0 * C * A * A / 1.7e8 + 4.0 * R * C / 2.0e8
 
 
-def job_device_bytes(R: int, C: int, A: int) -> int:
+def job_device_bytes(R: int, C: int, A: int, irreversible: bool = False) -> int:
     """Device footprint estimate of one in-flight job (bytes): plan tables,
     tokens, outputs and the plan's scratch (per-branch staging of the
-    large-alphabet Counts path, capped per plan; slot scratch otherwise)."""
+    large-alphabet Counts path, capped per plan; slot scratch otherwise).
+    Irreversible models at A = 16, 20, 32 stage the projected vectors beside
+    the raw ones: up to 2 A floats per vector, in blocks of at least 8 columns
+    padded by 2."""
     tables = 4 * R * (A + 1) * A * 6 + 4 * R * (A + 1) * (A * A + 4) * (A <= 8)
     tokens = 4 * R * C
     outputs = 4 * C * (A * A + A + 1)
-    if A >= 16:
-        scratch = min(STAGE_CAP, 8 * (R - 1) * A * C) + 4 * R * (A + 1) * min(C, 152 * 128)
+    if A >= 16 or irreversible:
+        staged = A + 2 * A * 10 // 8 if irreversible and A in (16, 20, 32) else A
+        scratch = min(STAGE_CAP, 8 * (R - 1) * staged * C) + 4 * R * (A + 1) * min(C, 152 * 128)
     elif A == 4:   # a node slot per step and resident column
         scratch = 10 * R * min(C, 152 * 768)
     else:
@@ -259,8 +263,8 @@ class Server:
     def _launch(self, job: Job, now: float):
         torch = self.torch
         R, C = job.RC
+        nbytes = self._bytes(job)
         A = len(ensure_diag(job.model).pi)
-        nbytes = job_device_bytes(R, C, A)
         slot = self.free_slots.pop()
         cost = job_cost_ms(R, C, A, job.f81)
         stream = (self.hi_streams if cost <= self.short_ms else self.streams)[slot]
@@ -344,6 +348,11 @@ class Server:
         self.used_bytes += nbytes
         self.inflight.append((job, slot, ev, nbytes, (None, d_aln, res, host, blocks)))
 
+    @staticmethod
+    def _bytes(job: Job) -> int:
+        m = ensure_diag(job.model)
+        return job_device_bytes(*job.RC, len(m.pi), is_irrev(m))
+
     def _cost(self, job: Job) -> float:
         c = getattr(job, "_cost_ms", None)
         if c is None:
@@ -352,9 +361,7 @@ class Server:
         return c
 
     def fits(self, job: Job) -> bool:
-        R, C = job.RC
-        A = len(ensure_diag(job.model).pi)
-        need = job_device_bytes(R, C, A)
+        need = self._bytes(job)
         if not self.free_slots:
             return False
         # long jobs may hold all but `short_slots` slots, so that short jobs
