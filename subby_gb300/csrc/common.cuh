@@ -4,7 +4,31 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
 namespace subby {
+
+// Lets kernel Fn ask for all the shared memory that a CTA can have, once per
+// device.  (Set before each launch to what that launch needs, the limit was
+// taken back by another host thread's call between the two, and the launch
+// failed.)
+template <auto Fn>
+cudaError_t allow_smem() {
+  static std::mutex m;
+  static uint64_t done = 0;   // a bit per device
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> g(m);
+  if (dev < 64 && (done >> dev & 1)) return cudaSuccess;
+  cudaFuncAttributes a{};
+  e = cudaFuncGetAttributes(&a, Fn);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(Fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+  if (e == cudaSuccess && dev < 64) done |= uint64_t(1) << dev;
+  return e;
+}
 
 // Step of the node schedule: one internal node p with children l < r.
 // Steps are stored in postorder (children before parents); the outside pass

@@ -278,8 +278,7 @@ template <int A, bool PB, bool CBUF>
 int cx_launch(const KParams &p, const float *sa, const float *sb, int c_base, int c_count, int n_lo, int n_hi,
               float2 *cbuf, int grid, cudaStream_t s) {
   const size_t smem = cx_smem<A>();
-  cudaError_t e =
-      cudaFuncSetAttribute(k_acc_cx<A, PB, CBUF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem<k_acc_cx<A, PB, CBUF>>();
   if (e != cudaSuccess) return (int)e;
   k_acc_cx<A, PB, CBUF><<<grid, kCxThreads, smem, s>>>(p, sa, sb, c_base, c_count, n_lo, n_hi, cbuf);
   return (int)cudaGetLastError();
@@ -296,7 +295,7 @@ int cx_launch_any(const KParams &p, bool pb, const float *sa, const float *sb, i
 template <int A>
 int bt_launch(const KParams &p, const float2 *cbuf, int c_base, int c_count, int row, int grid, cudaStream_t s) {
   const size_t smem = (size_t)3 * A * A * sizeof(double2) + (size_t)A * A * sizeof(float2);
-  cudaError_t e = cudaFuncSetAttribute(k_bt_cx<A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem<k_bt_cx<A>>();
   if (e != cudaSuccess) return (int)e;
   k_bt_cx<A><<<grid, 1024, smem, s>>>(p, cbuf, c_base, c_count, row);  // 32 warps: FP64 latency
   return (int)cudaGetLastError();

@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kFT, 1)
 
 int launch_acc_f81_64(const KParams &p, const float *sa, const float *sb, const float2 *sc, int c_base, int c_count,
                       int grid, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_acc_f81, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFBytes);
+  cudaError_t e = allow_smem<k_acc_f81>();
   if (e != cudaSuccess) return (int)e;
   k_acc_f81<<<grid, kFT, kFBytes, s>>>(p, sa, sb, sc, c_base, c_count);
   return (int)cudaGetLastError();

@@ -328,7 +328,7 @@ int accx(const KParams &p, const CxUnits &cu, const CxHost &h, const float *sa, 
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   const size_t smem = accx_floats(A, cu.UP, cu.G) * sizeof(float);
-  e = cudaFuncSetAttribute(k_accx<A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  e = allow_smem<k_accx<A>>();
   if (e != cudaSuccess) return (int)e;
   const int nblk = (c_count + cu.G - 1) / cu.G;
   k_accx<A><<<std::max(1, std::min(nblk, nsm)), 256, smem, s>>>(p, cu, pa, pb, c_base, c_count);

@@ -651,8 +651,7 @@ int acc_launch1(const KParams &p, const float *sa, const float *sb, int c_base, 
   const size_t smem = TCB ? (size_t)acc_vv_offset<A>() * sizeof(float) + 49152
                           : (size_t)(AccRing<A, Q>::SCAL + 2 * Gm::G + 2 * A * A + A + 2 * Gm::G * A + Gm::G) *
                                 sizeof(float);
-  cudaError_t e =
-      cudaFuncSetAttribute(k_acc<A, F81, TCB, PB, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem<k_acc<A, F81, TCB, PB, Q>>();
   if (e != cudaSuccess) return (int)e;
   k_acc<A, F81, TCB, PB, Q><<<grid, 256, smem, s>>>(p, sa, sb, c_base, c_count);
   return (int)cudaGetLastError();

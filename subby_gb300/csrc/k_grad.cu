@@ -286,7 +286,7 @@ int xgram_wide(const KParams &p, const float *sa, const float *sb, const float *
                int nsm, cudaStream_t s) {
   using G = XG<A>;
   const size_t smem = (size_t)G::FLOATS * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(k_xgram_wide<A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem<k_xgram_wide<A>>();
   if (e != cudaSuccess) return (int)e;
   const int items = ((p.R - 1 + G::NB - 1) / G::NB) * ((c_count + kXCols - 1) / kXCols);
   k_xgram_wide<A><<<std::max(1, std::min(items, 2 * nsm)), kXThreads, smem, s>>>(sa, sb, g, c_base, c_count, p.R, X,
@@ -299,7 +299,7 @@ int xgram_wide(const KParams &p, const float *sa, const float *sb, const float *
 int launch_xform(double *X, const double *tab64, int R, int A, double *grad_t, double *Cg, const int *err,
                  cudaStream_t s) {
   const size_t smem = (size_t)(A * A + A) * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(k_xform, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem<k_xform>();
   if (e != cudaSuccess) return (int)e;
   k_xform<<<R - 1, 256, smem, s>>>(X, tab64, R, A, grad_t);
   e = cudaGetLastError();

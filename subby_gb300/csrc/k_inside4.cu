@@ -176,7 +176,7 @@ size_t inside4_smem(int R, int nsteps, int nslots, int block, int per) {
 
 int launch_inside4(const KParams &p, int per, int grid, int block, size_t smem, cudaStream_t s) {
   auto fn = per == 2 ? k_inside4<2> : k_inside4<1>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = per == 2 ? allow_smem<k_inside4<2>>() : allow_smem<k_inside4<1>>();
   if (e != cudaSuccess) return (int)e;
   fn<<<grid, block, smem, s>>>(p);
   return (int)cudaGetLastError();

@@ -641,7 +641,7 @@ __global__ void __launch_bounds__(kPackBlock, 2) k_pass4_packed(const P4Queue Q)
 
 template <bool F, int M>
 int packed(const P4Queue &q, int grid, size_t smem, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_pass4_packed<F, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem<k_pass4_packed<F, M>>();
   if (e != cudaSuccess) return (int)e;
   k_pass4_packed<F, M><<<grid, kPackBlock, smem, s>>>(q);
   return (int)cudaGetLastError();
@@ -654,7 +654,7 @@ int pass4_s(const KParams &p, const A4Const &w, const int4 *prog, const int *oth
   std::copy(prog, prog + p.nsteps, T.step);
   std::copy(other, other + p.nsteps, T.other);
   auto fn = per == 2 ? k_pass4<F81, MASK, OUT, 2, S> : k_pass4<F81, MASK, OUT, 1, S>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = per == 2 ? allow_smem<k_pass4<F81, MASK, OUT, 2, S>>() : allow_smem<k_pass4<F81, MASK, OUT, 1, S>>();
   if (e != cudaSuccess) return (int)e;
   fn<<<grid, block, smem, s>>>(p, w, T);
   return (int)cudaGetLastError();

@@ -615,7 +615,7 @@ int qocc() {
   if (nb) return nb;
   const size_t smem = QG<A, CPL>::smem(F);
   auto fn = k_qwalk<A, CPL, F, M, MINB>;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+  if (allow_smem<k_qwalk<A, CPL, F, M, MINB>>() != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, q_threads<CPL, F>(), smem) != cudaSuccess || nb < 1)
     return 1;
   cached.store(nb);
@@ -625,8 +625,7 @@ int qocc() {
 template <int A, int CPL, bool F, int M, int MINB>
 int qlaunch(const KParams &p, float *sa, float *sb, int flags, int c_base, int c_count, int grid, cudaStream_t s) {
   const size_t smem = QG<A, CPL>::smem(F);
-  cudaError_t e =
-      cudaFuncSetAttribute(k_qwalk<A, CPL, F, M, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem<k_qwalk<A, CPL, F, M, MINB>>();
   if (e != cudaSuccess) return (int)e;
   k_qwalk<A, CPL, F, M, MINB><<<grid, q_threads<CPL, F>(), smem, s>>>(p, sa, sb, flags, c_base, c_count);
   return (int)cudaGetLastError();

@@ -547,11 +547,8 @@ __global__ void __launch_bounds__(128) k_small(const KParams P) {
 
 template <int A>
 int launch_t(const KParams &p, int grid, int block, size_t smem, cudaStream_t s) {
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_small<A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return (int)e;
-  }
+  cudaError_t e = allow_smem<k_small<A>>();
+  if (e != cudaSuccess) return (int)e;
   k_small<A><<<grid, block, smem, s>>>(p);
   return (int)cudaGetLastError();
 }

@@ -653,8 +653,7 @@ __global__ void __launch_bounds__(256, 1) k_tree(const KParams P) {
 
 template <int A, int ST>
 int tlaunch(const KParams &p, int grid, int block, size_t smem, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_tree<A, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+  cudaError_t e = allow_smem<k_tree<A, ST>>();
   if (e != cudaSuccess) return (int)e;
   k_tree<A, ST><<<grid, block, smem, s>>>(p);
   return (int)cudaGetLastError();

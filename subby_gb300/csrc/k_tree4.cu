@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(256, 1) k_tree4(const KParams P) {
 
 template <bool F, int M, int O>
 int t4launch(const KParams &p, int grid, int block, size_t smem, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_tree4<F, M, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem<k_tree4<F, M, O>>();
   if (e != cudaSuccess) return (int)e;
   k_tree4<F, M, O><<<grid, block, smem, s>>>(p);
   return (int)cudaGetLastError();

@@ -485,11 +485,8 @@ __global__ void __launch_bounds__(128) k_warp(const KParams P) {
 
 template <int A>
 int wlaunch_t(const KParams &p, int grid, int block, size_t smem, cudaStream_t s) {
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_warp<A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return (int)e;
-  }
+  cudaError_t e = allow_smem<k_warp<A>>();
+  if (e != cudaSuccess) return (int)e;
   k_warp<A><<<grid, block, smem, s>>>(p);
   return (int)cudaGetLastError();
 }

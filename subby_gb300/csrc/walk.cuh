@@ -1062,8 +1062,7 @@ int walk_launch_nd(const KParams &p, float *sa, float *sb, int c_base, int c_cou
   const int threads = 128 * Geo<A>::H;
   const size_t dyn = TC ? kTcDyn + 1024 + 8 * kRowBuf : 0;
   if (TC) {
-    cudaError_t e = cudaFuncSetAttribute(k_walk<A, MODE, TC, F81M, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)dyn);
+    cudaError_t e = allow_smem<k_walk<A, MODE, TC, F81M, ND>>();
     if (e != cudaSuccess) return (int)e;
   }
   k_walk<A, MODE, TC, F81M, ND><<<grid, threads, dyn, s>>>(p, sa, sb, c_base, c_count);
