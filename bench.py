@@ -531,7 +531,7 @@ def precision64_bench(args):
 def f81_64_bench(args):
     """A=64 F81 model (pi ~ Dirichlet(1^64)), the precision64 tree (R=127),
     C=65536 simulated columns: F81 fast-path Counts (closed-form walk and
-    tensor-core accumulation) and eigen-path Counts of the same model."""
+    FP32 accumulation) and eigen-path Counts of the same model."""
     import torch
     import oracle
     import subby_gb300 as sg
@@ -552,7 +552,7 @@ def f81_64_bench(args):
     ms_eig = _time_fn(lambda: plan.run(d_aln, loglike=False, counts=True, out=out), args.steps, args.warmup)
     print(json.dumps({"metric": "F81 fast-path Counts columns/s (A=64 F81, R=127, C=65536)", "value": C / (ms_f81 / 1e3),
                       "unit": UNIT, "ms_per_step": ms_f81, "steps": args.steps, "warmup": args.warmup,
-                      "higher_is_better": True, "dtype": "fp32 (split-bf16 tensor-core G accumulation)",
+                      "higher_is_better": True, "dtype": "fp32",
                       "err_vs_oracle_colwise_16cols": err,
                       "eigen_path_same_model": {"value": C / (ms_eig / 1e3), "ms_per_step": ms_eig}}))
     return 0

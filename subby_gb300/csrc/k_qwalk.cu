@@ -49,7 +49,7 @@ struct QG {
   static constexpr int N = SPL * CPL;                             // floats per lane and vector
   static constexpr int W = 8 * CPL;                               // columns per warp
   static constexpr int TILE = W * kQW;                            // columns per CTA
-  static constexpr int XS = CPL == 4 ? 32 : CPL == 2 ? 20 : 10;   // x rows: conflict-free strides
+  static constexpr int XS = CPL == 2 ? 20 : 10;                   // x rows: conflict-free strides
   static constexpr int BLK = (A + 1) * A;                         // floats of a ring block
   static constexpr int SLOT4 = (N + 3) / 4 * 32;                  // float4s of a warp's slot vector
   static constexpr size_t smem(bool f81m) {
@@ -185,7 +185,8 @@ __global__ void __launch_bounds__((q_threads<CPL, F81M>()), MINB)
   // steps forwards, then backwards).  One thread refills it: with one column
   // per lane a warp of its own, which never makes the column warps wait for
   // an issue slot; otherwise thread 0, one step at a time, into the stage of
-  // the step kQS - 1 ahead (its previous use is one step back).
+  // the step kQS - 2 ahead (its previous use is two steps back, which every
+  // warp has mostly left).
   const uint32_t per_tile = (MODE == 0 ? 1 : 2) * (uint32_t)nst;
   const uint32_t nring =
       F81M || (int)blockIdx.x >= ntiles ? 0 : per_tile * (uint32_t)((ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1);
@@ -277,8 +278,7 @@ __global__ void __launch_bounds__((q_threads<CPL, F81M>()), MINB)
 #pragma unroll
       for (int i = 0; i < SPL; ++i) {
         float *d = xb + qstate<A>(i, sg) * G::XS + CPL * cg;
-        if constexpr (CPL == 4) *reinterpret_cast<float4 *>(d) = make_float4(x.get(0, i), x.get(1, i), x.get(2, i), x.get(3, i));
-        else if constexpr (CPL == 2) *reinterpret_cast<float2 *>(d) = make_float2(x.get(0, i), x.get(1, i));
+        if constexpr (CPL == 2) *reinterpret_cast<float2 *>(d) = make_float2(x.get(0, i), x.get(1, i));
         else *d = x.get(0, i);
       }
       __syncwarp();
@@ -290,10 +290,7 @@ __global__ void __launch_bounds__((q_threads<CPL, F81M>()), MINB)
         m.row(0, T + j * A, sg);
         float xj[CPL];
         const float *xp = xb + j * G::XS + CPL * cg;
-        if constexpr (CPL == 4) {
-          const float4 t = *reinterpret_cast<const float4 *>(xp);
-          xj[0] = t.x, xj[1] = t.y, xj[2] = t.z, xj[3] = t.w;
-        } else if constexpr (CPL == 2) {
+        if constexpr (CPL == 2) {
           const float2 t = *reinterpret_cast<const float2 *>(xp);
           xj[0] = t.x, xj[1] = t.y;
         } else {

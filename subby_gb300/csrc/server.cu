@@ -70,10 +70,12 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
-// Kernel time per (column x tree node), ns, of Counts by path on GB300
-// (measured: A = 4 R = 255, A = 20 R = 399, A = 64 R = 127 workloads), plus
-// the host-link time of the job's tokens and results; used only to order
-// and slice work, never to skip any.
+// Estimated kernel time per (column x tree node), ns, of Counts by path on
+// GB300, plus the host-link time of the job's tokens and results; used only to
+// order, pack and slice work, never to skip any.  (The kernels now measure
+// 0.008 at A = 4, R = 255, 0.22 at A = 20, R = 199, 0.94 and 0.54 with F81 at A
+// = 64, R = 127; the values are those that short_ms and slice_ms were set
+// with.)
 double ns_per_col_node(int A, bool f81) {
   if (A <= 8) return f81 ? 0.011 : 0.012;
   if (A <= 20) return f81 ? 0.10 : 0.30;

@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
     };
 
     // ---------------------------------------------------------------- inside
-    constexpr bool kEarlyB = TC && MODE == 1 && ND && !f81m;
+    constexpr bool kEarlyB = TC && MODE == 1 && ND;
     BV<A> ur;
     int eRoot = 0, iRoot = 0;
     if (P.root_is_leaf) {
@@ -866,6 +866,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
       if (leafcode >= 0) wk.st_code(pb, nrows, Ut + 32 * h, leafcode);
     };
     constexpr bool kFuse = TC && MODE == 1;
+    static_assert(!kFuse || !F81M, "the tensor-core staging is of the general products");
     // Leaf branches of the derived-node-free instance: a step's products are
     // issued together and read in the next step, after its loads.
     bool pend_l = false, pend_r = false;
@@ -935,13 +936,8 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
         wk.obs(U, codep);
         const int eUp = nl.e + nr.e + wk.rescale(U);
         if constexpr (kFuse) {
-          if constexpr (f81m) {
-            mprod(O, D, s0.x, true);
-            emit_tc(s0.x, D, &U, -1, eD + eUp, actp, Onone, nullptr);
-          } else {
-            if constexpr (kEarlyB) flush();
-            emit_tc(s0.x, D, &U, -1, eD + eUp, actp, O, P.tab16 + (size_t)s0.x * 24576 + 12288, kEarlyB);
-          }
+          if constexpr (kEarlyB) flush();
+          emit_tc(s0.x, D, &U, -1, eD + eUp, actp, O, P.tab16 + (size_t)s0.x * 24576 + 12288, kEarlyB);
         } else if constexpr (MODE == 3) {
           mprod(O, D, s0.x, true);
           emit(s0.x, D, U, -1, eD + eUp, actp, &O);
@@ -997,8 +993,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
             wk.obs(du, dcode);
             wk.rescale(du);  // same exponent as in the gather: eU_c = me.e
             if constexpr (kFuse) {
-              if constexpr (f81m) emit_tc(sc.x, Dc, &du, -1, eDc + me.e, actc, Onone, nullptr);
-              else emit_tc(sc.x, Dc, &du, -1, eDc + me.e, actc, Oc, P.tab16 + (size_t)sc.x * 24576 + 12288);
+              emit_tc(sc.x, Dc, &du, -1, eDc + me.e, actc, Oc, P.tab16 + (size_t)sc.x * 24576 + 12288);
             } else if constexpr (MODE == 3) {
               mprod(Oc, Dc, sc.x, true);
               emit(sc.x, Dc, du, -1, eDc + me.e, actc, &Oc);
@@ -1006,7 +1001,7 @@ __global__ void __launch_bounds__(128 * Geo<A>::H, 1) k_walk(const KParams P, fl
               emit(sc.x, Dc, du, -1, eDc + me.e, actc);
             }
           }
-          if constexpr ((!kFuse || f81m) && MODE != 3) mprod(Oc, Dc, sc.x, true);
+          if constexpr (!kFuse && MODE != 3) mprod(Oc, Dc, sc.x, true);
           wk.obs(Oc, dcode);
           const int eOc = eDc + wk.rescale(Oc);
 #pragma unroll

@@ -118,8 +118,10 @@ def _plan_key(tree, model):
 
 STAGE_CAP = 4 << 30   # per-plan staging cap of the large-alphabet path (bytes)
 
-# Device time per (column x tree node), ns, by path (GB300, Counts): used only
-# to order and slice work, never to skip any.
+# Estimated device time per (column x tree node), ns, by path (GB300, Counts):
+# used only to order and slice work, never to skip any.  (The kernels have
+# become faster since: 0.008 at A = 4, 0.22 at A = 20, 0.94 and 0.54 with F81 at
+# A = 64; the values are those that short_ms and slice_ms were set with.)
 _NS_PER_COL_NODE = {("4", False): 0.012, ("4", True): 0.011, ("16", False): 0.30, ("16", True): 0.10,
                     ("64", False): 1.2, ("64", True): 0.70}
 
