@@ -32,7 +32,9 @@
  *    pointers on the current device.  With host pointers the call copies in
  *    and out on `stream` and returns after the results are in host memory;
  *    with device pointers it only enqueues work on `stream` (NULL = legacy
- *    default stream).
+ *    default stream).  Calls of one plan may come from several threads and go
+ *    to several streams; those that use the plan's workspace wait on the
+ *    device for one another.
  *  - Every function returns 0 (SUBBY_OK) or a negative SUBBY_ERR_* code;
  *    subby_strerror() names it and subby_last_error() gives details of the
  *    most recent failure on the calling thread.

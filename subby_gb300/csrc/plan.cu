@@ -504,6 +504,10 @@ double cx_cond(const IrrevInput &ir, int A) {
   return cond;
 }
 
+// Least probability (times pi) of a change along a branch in the closed form
+// of F81 / JC models: about the rounding of an FP64 sum.
+constexpr float kLeastChange = 1.3877788e-17f;   // 2^-56
+
 // Eigensystems up to this condition number take the paired units.  Rounding of
 // the FP32 projections is amplified by it on the way back: the counts of the
 // paired and of the general form (k_acc_cx) differ by 3e-7 times the condition
@@ -776,7 +780,10 @@ int plan_create(const int32_t *parent, const double *dist, const double *evals, 
     f[2] = (float)(t * (1.0 + e) - 2.0 * pp / mu81);
     f[3] = (float)t;
     hef[2 * n] = (float)e;
-    hef[2 * n + 1] = (float)(-std::expm1(-mu81 * t));
+    // (never exactly 0: the general tables, FP64 sums over the eigensystem,
+    // hold their rounding at t = 0, and a column whose leaves contradict one
+    // another on branches of length 0 keeps finite counts with them)
+    hef[2 * n + 1] = std::max((float)(-std::expm1(-mu81 * t)), kLeastChange);
     for (int k = 0; k < A; ++k) at(o.ME + n * A + k) = (float)(evals[k] * E[k]);
   }
   std::vector<double> S64((size_t)A * A);
