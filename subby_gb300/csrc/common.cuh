@@ -69,7 +69,7 @@ struct TableOffsets {
   int S;     // A x A         : S[i][j] = sum_k V_ik mu_k V_jk
   int ME;    // R x A         : mu_k e^{mu_k t_n} (distance gradient)
   int K;     // R x (A+1) x A x A (A <= 8 only): K[n][code][k][l] = J[n][k][l] Ut[code][l]
-  int EF;    // R x 2         : e^{-mu t_n}, 1 - e^{-mu t_n} (F81 closed form of M(t))
+  int EF;    // R x 2         : e^{-mu t_n}, 1 - e^{-mu t_n} (at least 2^-56; F81 closed form of M(t))
   int total;
 };
 

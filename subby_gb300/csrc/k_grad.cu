@@ -92,7 +92,8 @@ __global__ void __launch_bounds__(kXThreads) k_xgram(const float *__restrict__ s
 // half a row): 4 + LW floats for 4 LW multiply-adds, and a CTA takes NB
 // branches of the same columns, whose rows come through a ring of bulk
 // copies.  The subsets are added in their order, as k_xgram does, so that the
-// gradients of up to 4096 columns are the same in every call.
+// gradients of up to 4096 columns are the same in every call (A = 20, R = 399,
+// 50000 columns, 3.2 GB: 735 us; with an FP64 atomic per entry and subset 823).
 template <int A>
 struct XG {
   static constexpr int LW = A == 32 ? 16 : A;
